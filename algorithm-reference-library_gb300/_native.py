@@ -63,6 +63,8 @@ SIGNATURES = {
                                              _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     'arlgpu_decoalesce': (ctypes.c_int, [_vp, _i64, _vp, _i32, _i32, _i32, _i32, ctypes.c_int, _vp, _vp, _vp]),
     'arlgpu_dft_predict': (ctypes.c_int, [_vp, _vp, _i64, _vp, _vp, _i32, _i32, _i32, ctypes.c_int, _vp, _vp]),
+    'arlgpu_row_channels_bytes': (ctypes.c_int, [_i32, _P(_sz)]),
+    'arlgpu_row_channels': (ctypes.c_int, [_vp, _i64, _i32, _vp, _vp, _vp, _sz, _vp]),
     'arlgpu_dft_adjoint': (ctypes.c_int, [_vp, _i64, _vp, _i32, _i32, ctypes.c_int, _vp, _vp, _vp]),
     'arlgpu_hogbom': (ctypes.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _f64, _f64, _i32, _f64, _f64, _f64,
                                      _vp, _vp, _P(_i32), _vp]),

@@ -7,10 +7,11 @@ Reference behaviour:
 
 Each component adds flux[chan(row), pol] * exp(-2 pi i uvw . s) to every row,
 s = (l, m, sqrt(1 - l^2 - m^2) - 1) with (l, m) the component's direction
-cosines relative to the visibility phase centre.  The phase is formed in FP64
-on the GPU (``csrc/dft.cu``).
+cosines relative to the visibility phase centre.  The phase is formed on the
+GPU in FP64, or modulo one turn in fixed point (``csrc/dft.cu``).
 """
 import collections.abc
+import ctypes
 
 import numpy
 import torch
@@ -41,6 +42,23 @@ def _row_channels(frequency):
     (``get_frequency_map`` with no image)."""
     uf, inv = numpy.unique(numpy.asarray(frequency), return_inverse=True)
     return inv.astype(numpy.int32), uf.size
+
+
+def _device_row_channels(frequency, max_chan, device):
+    """(channel of each row, number of channels) as ``_row_channels``, for rows on
+    the device; the number is only known to exceed ``max_chan`` when it does."""
+    if max_chan > 1 << 14:  # the device table's limit
+        rc, nchan = _row_channels(frequency.cpu().numpy())
+        return torch.as_tensor(rc, device=device), nchan
+    f = frequency.to(device=device, dtype=torch.float64).contiguous()
+    nbytes = ctypes.c_size_t(0)
+    nat.call('arlgpu_row_channels_bytes', max_chan, ctypes.byref(nbytes))
+    ws = torch.empty(nbytes.value, dtype=torch.uint8, device=device)
+    rc = torch.empty(f.shape[0], dtype=torch.int32, device=device)
+    nchan = torch.empty(1, dtype=torch.int32, device=device)
+    nat.call('arlgpu_row_channels', nat.ptr(f), f.shape[0], max_chan, nat.ptr(rc), nat.ptr(nchan), nat.ptr(ws),
+             ws.numel(), nat.stream_ptr())
+    return rc, int(nchan.item())
 
 
 def dft_predict(uvw, row_chan, lmn, flux, vis, precision):
@@ -77,10 +95,8 @@ def predict_skycomponent_visibility(vis, sc, precision=None):
     lmn_t = torch.as_tensor(lmn, device=device)
     if isinstance(vis, DeviceVisibility):
         prec = vis.precision
-        freq = vis.frequency.cpu().numpy()
-        rc, nchan = _row_channels(freq)
+        rc_t, nchan = _device_row_channels(vis.frequency, flux.shape[1], device)
         assert flux.shape[1] >= nchan and flux.shape[2] == vis.npol, "component and visibility channels / pols"
-        rc_t = torch.as_tensor(rc, device=device)
         flux_t = torch.as_tensor(numpy.ascontiguousarray(flux), device=device)
         dft_predict(vis.uvw, rc_t, lmn_t, flux_t, vis.vis, prec)
         return vis

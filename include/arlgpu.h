@@ -301,10 +301,19 @@ int arlgpu_decoalesce(const void *rows, int64_t nrows, const int64_t *cindex, in
  *   [ncomp][nchan][npol] float64, vis [nvis][npol] complex of the precision (updated in
  *   place).  row_chan [nvis] int32 may be NULL when nchan == 1.  Phases in FP64.
  * arlgpu_dft_adjoint: image[k][p] += Re sum_r conj(exp(-2 pi i uvw_r . lmn_k)) x[r][p], the
- *   adjoint for one channel (no reference counterpart; the dense gradient reference). */
+ *   adjoint for one channel (no reference counterpart; the dense gradient reference).
+ * arlgpu_row_channels: row_chan[r] = the rank of frequency[r] among the rows' distinct
+ *   frequencies, ascending (get_frequency_map with no image,
+ *   processing_library/imaging/imaging_params.py:18-48), and *nchan_dev (device) their
+ *   number; with more than max_chan (at most 2^14) of them *nchan_dev is only known to be
+ *   larger than max_chan and row_chan is not meaningful.  Device workspace of
+ *   arlgpu_row_channels_bytes, 8-byte aligned. */
 int arlgpu_dft_predict(const double *uvw, const int32_t *row_chan, int64_t nvis, const double *lmn,
                        const double *flux, int32_t ncomp, int32_t nchan, int32_t npol, int precision, void *vis,
                        void *stream);
+int arlgpu_row_channels_bytes(int32_t max_chan, size_t *bytes_host);
+int arlgpu_row_channels(const double *frequency, int64_t nvis, int32_t max_chan, int32_t *row_chan,
+                        int32_t *nchan_dev, void *workspace, size_t workspace_bytes, void *stream);
 int arlgpu_dft_adjoint(const double *uvw, int64_t nvis, const double *lmn, int32_t ncomp, int32_t npol,
                        int precision, const void *x, double *image, void *stream);
 
