@@ -59,6 +59,14 @@ __device__ __forceinline__ void st_map16(RowMap *p, const RowMap &m) {
 // of an 8-wide window (PSWF support 8) on distinct banks.
 __host__ __device__ constexpr int fx_pitch(int sg) { return sg % 32 == 0 ? sg + 8 : sg; }
 
+// One axis of the integer mapping (fix_value in mapping.cuh): |scale| 2^20 as
+// rhi 2^32 + rlo in units of 2^-(64 - shift of x), its sign, and the constant term.
+struct FixAxis {
+  uint32_t rhi, rlo;
+  int32_t s0, neg;
+  int64_t c;
+};
+
 struct Geom {
   int32_t nchan, npol, nw, ny, nx;     // grid
   int32_t cf_nchan, cf_npol, nz, O, S; // cf
@@ -78,6 +86,9 @@ struct Geom {
   // Fixed-point decisions (pow2O and every limit below 2^29): the tolerances
   // above in units of 2^-20, plus one.
   int32_t fixmap, tq_u, tq_v, tq_w, tq_z, tq_f;
+  // The same decisions with X and P formed in integers (fixint: every axis fits)
+  int32_t fixint;
+  FixAxis fu, fv, fw, fz, ff;
   // One grid w-plane whose interval contains every cf plane's (w-projection),
   // or one cf plane whose interval contains every grid plane's (w-stacking,
   // 2-D): that index is 0 for every row the other axis accepts, so the fast
@@ -87,6 +98,7 @@ struct Geom {
   int32_t T;       // tile edge (grid pixels)
   int32_t SG;      // staged subgrid edge = T + S
   int32_t ntu, ntv;
+  uint32_t rcpT;   // ceil(2^32 / T): pixel / T as a high word (exact below 2^20 pixels)
   uint32_t nbins;  // nchan * nw * ntv * ntu; key == nbins marks a rejected row
 };
 

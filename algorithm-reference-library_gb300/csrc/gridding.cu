@@ -2412,6 +2412,30 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
     g->fixmap = g->pow2O && g->Xlim_u < lim && g->Xlim_v < lim && g->Plim_w < lim && g->Plim_z < lim &&
                 g->Plim_f < lim && g->tq_u < (1 << 18) && g->tq_v < (1 << 18) && g->tq_w < (1 << 18) &&
                 g->tq_z < (1 << 18) && g->tq_f < (1 << 18);
+    // Integer form: axis value = x scale + c, x up to twice the grid's largest
+    // |x| below 2^63, |scale| 2^20 in the remaining 64 bits' product.
+    auto fit = [](double scale, double c, double n, FixAxis *a) {
+      const double xmax = (fabs(n) + fabs(c)) / fabs(scale);
+      // x scale + c stays below 2^31 up to 4 xmax, and |scale| 2^(84 - S) below 2^52
+      if (!(xmax > 0.0) || !std::isfinite(xmax) || !(fabs(n) + fabs(c) < 268435456.0)) return false;
+      int e;
+      frexp(xmax, &e);             // xmax < 2^e
+      const int S = 62 - e;        // |x| 2^S < 2^63 up to 2 xmax
+      if (S > 900 || S < -900) return false;
+      const uint64_t R = (uint64_t)(ldexp(fabs(scale), 84 - S) + 0.5);
+      a->rhi = (uint32_t)(R >> 32);
+      a->rlo = (uint32_t)R;
+      a->s0 = 1085 - S;
+      a->neg = scale < 0.0;
+      a->c = (int64_t)llround(c * 1048576.0);
+      return true;
+    };
+    auto plane = [&](const arlgpu_axis &a, double r, int n, FixAxis *o) {
+      return fit(r, a.crpix - 1.0 - a.crval * r, (double)n + 2.0, o);
+    };
+    g->fixint = g->fixmap && fit(g->rOu, g->cOu, g->Xlim_u, &g->fu) && fit(g->rOv, g->cOv, g->Xlim_v, &g->fv) &&
+                (g->skip_zg || plane(gd->w, g->rcp_gw, gd->nw, &g->fw)) &&
+                (g->skip_zc || plane(cd->z, g->rcp_cz, cd->nz, &g->fz)) && plane(gd->f, g->rcp_gf, gd->nchan, &g->ff);
   }
   // Subgrid edge: 64 cells when npol planes of it (with the FP32 compensation
   // words) fit in 64 KiB of shared memory, else 32.
@@ -2428,6 +2452,7 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
                 g->S, g->npol);
   g->SG = SG;
   g->T = SG - g->S;
+  g->rcpT = (uint32_t)(((1ull << 32) + g->T - 1) / g->T);
   g->ntu = (g->nx + g->T - 1) / g->T;
   g->ntv = (g->ny + g->T - 1) / g->T;
   uint64_t nb = (uint64_t)g->nchan * g->nw * g->ntv * g->ntu;
