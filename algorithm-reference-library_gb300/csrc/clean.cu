@@ -5,32 +5,24 @@
 //   hogbom_complex            processing_library/arrays/cleaners.py:72-131
 //   deconvolve_cube('hogbom') processing_components/image/deconvolution.py:43-300
 //
-// Each minor-cycle iteration is two launches on one stream, with no host
-// round trip:
-//   k_hog_find  argmax of |res * window| (or |res|) over the image, first
-//               index on ties as numpy.argmax; the last block to finish
-//               (counted with an atomic, no waiting) reduces the per-block
-//               maxima, forms mval = res[peak] * gain / pmax and adds it to the
-//               component image;
-//   k_hog_sub   res[overlap] -= psf[overlap] * mval, and the stopping test
-//               |res[peak]| < 0.9 * threshold on the updated peak.
+// The real minor cycle is one cooperative launch (k_hogbom below); the complex
+// and multi-scale ones are two launches per iteration on one stream, with no
+// host round trip:
+//   k_*_find  argmax over the image, first index on ties as numpy.argmax; the
+//             last block to finish (counted with an atomic, no waiting) reduces
+//             the per-block maxima and forms the component;
+//   k_*_sub   the PSF patch subtracted, and the stopping test on the peak.
 // A set stop flag turns the remaining launches into no-ops; the host reads
 // the flag every kCheck iterations to stop launching.  All arithmetic is FP64
 // with each operation rounded on its own (no FMA contraction), in the
 // reference's order, so the result equals NumPy's bit for bit.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace arlgpu {
 
 void count_launch(unsigned n);
-
-struct HogState {
-  double mval;
-  long long peak;  // flat index of the peak, row-major [nx][ny]
-  int stop;
-  int iters;
-  unsigned int counter;
-};
 
 struct Best {
   double v;
@@ -45,91 +37,355 @@ __device__ __forceinline__ Best better(Best a, Best b) {
 
 constexpr int kFindThreads = 256;
 
-__global__ void __launch_bounds__(kFindThreads)
-k_hog_find(const double *__restrict__ res, const double *__restrict__ window, long long n, double gain, double pmax,
-           double *__restrict__ comps, Best *__restrict__ partial, HogState *__restrict__ st) {
-  if (st->stop) return;
-  __shared__ Best s_best[kFindThreads / 32];
-  __shared__ bool s_last;
-  Best b{-1.0, 0x7fffffffffffffffll};
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double a = window ? fabs(__dmul_rn(res[i], window[i])) : fabs(res[i]);
-    b = better(b, Best{a, i});
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    Best c;
-    c.v = __shfl_xor_sync(0xffffffffu, b.v, o);
-    c.i = __shfl_xor_sync(0xffffffffu, b.i, o);
-    b = better(b, c);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) s_best[warp] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    Best t = s_best[0];
-    for (int k = 1; k < kFindThreads / 32; ++k) t = better(t, s_best[k]);
-    partial[blockIdx.x] = t;
-    __threadfence();
-    s_last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  // Last block: reduce the per-block maxima.
-  __threadfence();
-  Best t{-1.0, 0x7fffffffffffffffll};
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-    Best q;  // other blocks' results: read past L1
-    q.v = __ldcg(&partial[k].v);
-    q.i = __ldcg(&partial[k].i);
-    t = better(t, q);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    Best c;
-    c.v = __shfl_xor_sync(0xffffffffu, t.v, o);
-    c.i = __shfl_xor_sync(0xffffffffu, t.i, o);
-    t = better(t, c);
-  }
-  if (lane == 0) s_best[warp] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    Best f = s_best[0];
-    for (int k = 1; k < kFindThreads / 32; ++k) f = better(f, s_best[k]);
-    const double mval = __ddiv_rn(__dmul_rn(res[f.i], gain), pmax);
-    comps[f.i] = __dadd_rn(comps[f.i], mval);
-    st->mval = mval;
-    st->peak = f.i;
-    st->counter = 0;
+// ---------------------------------------------------------------------------
+// Hogbom minor cycle, all iterations in one cooperative launch.
+//
+// As two launches per iteration (a search over the whole image, a subtraction)
+// an iteration on 1024^2 with a 512^2 PSF took 22 us of GPU time and 30 us in
+// all: the search alone spends three FP64 operations a pixel at 2 a clock and
+// SM, and a launch costs more than the subtraction.  Here
+//   * the image is cut into segments of 256 pixels of one row, dealt to the CTAs
+//     in turn (an odd number of CTAs, so that a patch narrower than the image
+//     still meets all of them); the residual stays in shared memory for the
+//     whole cycle where it fits (about 2048^2), else in its global array;
+//   * each segment's best pixel is kept, and only the segments that the PSF patch
+//     touched are searched again, while they are updated.  |res * window| is
+//     compared as integers, and a window of 0 or 1 (2-bit codes) takes no product;
+//   * an iteration has one exchange: every CTA publishes its best pixel in a
+//     16-byte slot and reads all the others', so all know the peak and need no
+//     second barrier.  Both words of a slot carry their own generation mark (two
+//     buffers in turn: nobody can be two iterations ahead), so that they need no
+//     fence.  The wait is bounded; when it runs out the cycle ends with an error.
+// What is left is the exchange (two L2 trips), one division and two FP64
+// operations per pixel of the patch: 5.7 us an iteration (3.8 on 128^2).
+// ---------------------------------------------------------------------------
+constexpr int kHogThreads = 512, kHogSeg = 256, kHogPx = kHogSeg / 32;
+constexpr unsigned long long kAbsMask = 0x7fffffffffffffffull;
+
+// Copies of the slots, each polled by every kHogCopies-th CTA: with one, the
+// 19 cache lines were read by all SMs at once and an iteration took 6.4 us on the
+// smallest image.
+constexpr int kHogCopies = 16;
+constexpr int kHogPoll = 5;         // slots a polling lane reads: up to 160 CTAs
+constexpr int kHogTries = 1 << 20;  // rounds of polling (about a microsecond each) before a CTA gives up
+
+// a / b for y = 1 / b rounded to nearest: after a correction step the quotient is
+// within an ulp, and after a second one it is the rounded quotient (Markstein, IBM
+// J. Res. Dev. 34, 1990, pp. 111-119).  Five dependent operations; the peak's
+// component is on every CTA's path.  Outside the range where no step under- or
+// overflows, the division itself.
+__device__ __forceinline__ double hog_quotient(double a, double b, double y) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+  if (ea < 1023 - 800 || ea > 1023 + 800 || eb < 1023 - 100 || eb > 1023 + 100) return __ddiv_rn(a, b);
+  double q = __dmul_rn(a, y);
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ void hog_put(unsigned long long *p, unsigned long long a, unsigned long long b) {
+  asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void hog_get(const unsigned long long *p, unsigned long long *a, unsigned long long *b) {
+  asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(*a), "=l"(*b) : "l"(p) : "memory");
+}
+
+struct HogStatus {
+  int iters, stop, error;
+};
+
+struct HogArgs {
+  const double *src, *psf, *window;
+  double *comps, *res;
+  long long nx, ny, pnx, pny;
+  double gain, pmax, stop_level;
+  int niter, width, nloc;       // iterations of this launch, pixels per segment, segments per CTA (at most)
+  unsigned long long *slots;    // [2][kHogCopies][gridDim.x][2]
+  unsigned char *bests;         // the segments' bests of all CTAs where they do not fit shared memory, else null
+  double *lookup;               // [2][gridDim.x]: the residual at a slot's pixel where |res| is not the slot's value
+  HogStatus *status;
+};
+
+// A candidate: |res * window| as its bit pattern, and the pixel; first index on
+// ties.  Where nothing qualifies (every value a NaN) the pixel stays kNoPixel.
+constexpr int kNoPixel = 0x7fffffff;
+__device__ __forceinline__ void hog_take(unsigned long long v, int i, unsigned long long *bv, int *bi) {
+  if (v > *bv || (v == *bv && i < *bi)) {
+    *bv = v;
+    *bi = i;
   }
 }
 
-// res[overlap] -= psf[overlap] * mval (overlapIndices of the reference), then
-// the stopping test on the updated peak.
-__global__ void k_hog_sub(double *__restrict__ res, int nx, int ny, const double *__restrict__ psf, int pnx, int pny,
-                          double stop_level, HogState *__restrict__ st) {
-  if (st->stop) return;
-  const long long peak = st->peak;
-  const int mx = (int)(peak / ny), my = (int)(peak - (long long)mx * ny);
-  const double mval = st->mval;
-  const int wx = pnx / 2, wy = pny / 2;
-  const int r0 = max(0, mx - wx), r1 = min(nx, mx + wx);
-  const int c0 = max(0, my - wy), c1 = min(my + wy, ny);
-  const int p0 = max(0, wx + (r0 - mx)), q0 = max(0, wy + (c0 - my));
-  const int p1 = min(pnx, wx + (r1 - mx)), q1 = min(wy + (c1 - my), pny);
-  // numpy slices of unequal length would raise; the extents agree for every
-  // peak inside the image, so the patch is (r1 - r0) x (c1 - c0)
-  const int h = min(r1 - r0, p1 - p0), w = min(c1 - c0, q1 - q0);
-  const long long total = (long long)h * w;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k / w), j = (int)(k - (long long)i * w);
-    const long long ri = (long long)(r0 + i) * ny + (c0 + j);
-    const double nv = __dsub_rn(res[ri], __dmul_rn(psf[(long long)(p0 + i) * pny + (q0 + j)], mval));
-    res[ri] = nv;
-    if (ri == peak) {
-      st->iters += 1;
-      if (fabs(nv) < stop_level) st->stop = 1;
+// The lane whose (v, key) is best: largest v, then smallest key.  Warp-wide
+// 32-bit maxima and minima, a word at a time.
+__device__ __forceinline__ bool hog_largest(unsigned long long v) {
+  const unsigned all = 0xffffffffu, vh = (unsigned)(v >> 32), vl = (unsigned)v;
+  const bool in = vh == __reduce_max_sync(all, vh);
+  return (__reduce_max_sync(all, in ? vl : 0u) == vl) && in;
+}
+__device__ __forceinline__ int hog_best_lane(unsigned long long v, unsigned key) {
+  const unsigned all = 0xffffffffu;
+  const bool in = hog_largest(v);
+  const unsigned k = __reduce_min_sync(all, in ? key : all);
+  return __ffs(__ballot_sync(all, in && key == k)) - 1;
+}
+__device__ __forceinline__ int hog_best_lane(unsigned long long v, unsigned long long key) {
+  const unsigned all = 0xffffffffu, kh = (unsigned)(key >> 32), kl = (unsigned)key;
+  bool in = hog_largest(v);
+  const unsigned h = __reduce_min_sync(all, in ? kh : all);
+  in = in && kh == h;
+  const unsigned l = __reduce_min_sync(all, in ? kl : all);
+  return __ffs(__ballot_sync(all, in && kl == l)) - 1;
+}
+
+// |res * window| of one pixel; NaN results never qualify (marked all ones).
+__device__ __forceinline__ unsigned long long hog_value(double r, int code, const double *win) {
+  unsigned long long a = (unsigned long long)__double_as_longlong(r) & kAbsMask;
+  if (code == 2) a = (unsigned long long)__double_as_longlong(__dmul_rn(r, *win)) & kAbsMask;
+  if (code == 0) a = a >= 0x7ff0000000000000ull ? ~0ull : 0;
+  return a > 0x7ff0000000000000ull ? ~0ull : a;
+}
+
+__device__ __forceinline__ int hog_code(const double *window, long long px) {
+  const unsigned long long w = (unsigned long long)__double_as_longlong(window[px]);
+  return w == 0x3ff0000000000000ull ? 1 : ((w & kAbsMask) == 0 ? 0 : 2);
+}
+
+template <bool SMEM> struct HogPx { using T = int; };
+template <> struct HogPx<true> { using T = unsigned short; };
+
+template <bool SMEM>
+__global__ void __launch_bounds__(kHogThreads, 1)
+k_hogbom(HogArgs a) {
+  extern __shared__ double s_dyn[];
+  __shared__ unsigned long long s_bits, s_key;  // the iteration's peak
+  __shared__ unsigned s_word;
+  __shared__ double s_mval;
+  __shared__ int s_stop, s_end;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x, cta = blockIdx.x;
+  const int width = SMEM ? kHogSeg : a.width;
+  // segments per row, in all (32-bit divisions below: the host keeps nseg below 2^31)
+  const unsigned spr = (unsigned)((a.ny + width - 1) / width), nseg = (unsigned)a.nx * spr;
+  // shared memory: [nloc][256] residual, [nloc][32] window codes (SMEM), then the segments' bests
+  double *s_res = s_dyn;
+  unsigned short *s_code = reinterpret_cast<unsigned short *>(s_dyn + (SMEM ? (size_t)a.nloc * kHogSeg : 0));
+  unsigned long long *s_segv =
+      reinterpret_cast<unsigned long long *>(s_dyn + (SMEM ? (size_t)a.nloc * (kHogSeg + 8) : 0));
+  if (!SMEM && a.bests) s_segv = reinterpret_cast<unsigned long long *>(a.bests + (size_t)cta * a.nloc * 16);
+  using Px = typename HogPx<SMEM>::T;
+  constexpr Px kNone = (Px)kNoPixel;
+  Px *s_segi = reinterpret_cast<Px *>(s_segv + a.nloc);
+
+  // Local pixel p of segment i: offset p in [0, width) of segment cta + i G.
+  // A segment's row: seg and spr stay below 2^15 where the residual is in shared memory, so that a high word does it.
+  const unsigned inv = SMEM && spr > 1 ? 0xffffffffu / spr + 1 : 0;
+  auto seg_div = [&](unsigned s) { return SMEM ? (spr > 1 ? __umulhi(s, inv) : s) : s / spr; };
+  auto seg_row = [&](int i, long long *col) {
+    const unsigned s = (unsigned)cta + (unsigned)i * G, row = seg_div(s);
+    *col = (long long)(s - row * spr) * width;
+    return (long long)row;
+  };
+  // Best pixel of segment i after subtracting mval * psf over columns [c0, c1) with the PSF pixel of column c at
+  // prow[c] (null: no subtraction).  pre: the warp's PSF values when they are already in registers.
+  auto scan = [&](int i, long long row, long long col, const double *prow, long long c0, long long c1, double mval,
+                  const double *pre) {
+    unsigned long long bv = 0;
+    int bi = kNoPixel;
+    const unsigned codes = SMEM && a.window ? s_code[i * 32 + lane] : 0x5555u;
+    auto one = [&](int j) {
+      const int p = lane + 32 * j;
+      const long long c = col + p, px = row * a.ny + c;
+      if (c >= a.ny) return;
+      double r = SMEM ? s_res[i * kHogSeg + p] : a.res[px];
+      if (prow && c >= c0 && c < c1) {
+        r = __dsub_rn(r, __dmul_rn(pre ? pre[j] : prow[c], mval));
+        if (SMEM)
+          s_res[i * kHogSeg + p] = r;
+        else
+          a.res[px] = r;
+      }
+      const int code = SMEM ? (codes >> (2 * j)) & 3 : (a.window ? hog_code(a.window, px) : 1);
+      const unsigned long long v = hog_value(r, code, a.window + px);
+      if (v != ~0ull) hog_take(v, p, &bv, &bi);
+    };
+    if (SMEM) {
+#pragma unroll
+      for (int j = 0; j < kHogPx; ++j) one(j);
+    } else {
+      for (int j = 0; j < width / 32; ++j) one(j);
     }
+    if (lane == hog_best_lane(bv, (unsigned)bi)) {
+      s_segv[i] = bv;
+      s_segi[i] = (Px)bi;
+    }
+  };
+
+  const int mine = (unsigned)cta < nseg ? (int)((nseg - 1 - cta) / G) + 1 : 0;
+  for (int i = warp; i < mine; i += kHogThreads / 32) {
+    long long col;
+    const long long row = seg_row(i, &col);
+    if (SMEM) {
+      unsigned codes = 0;
+#pragma unroll
+      for (int j = 0; j < kHogPx; ++j) {
+        const long long c = col + lane + 32 * j;
+        const bool in = c < a.ny;
+        s_res[i * kHogSeg + lane + 32 * j] = in ? a.src[row * a.ny + c] : 0.0;
+        codes |= (in && a.window ? hog_code(a.window, row * a.ny + c) : 1) << (2 * j);
+      }
+      s_code[i * 32 + lane] = (unsigned short)codes;
+    } else if (a.src != a.res) {
+      for (int p = lane; p < width && col + p < a.ny; p += 32) a.res[row * a.ny + col + p] = a.src[row * a.ny + col + p];
+    }
+    scan(i, row, col, nullptr, 0, 0, 0.0, nullptr);
   }
+  const long long wx = a.pnx / 2, wy = a.pny / 2;
+  const double centre = a.psf[wx * a.pny + wy], rcp = __drcp_rn(a.pmax);
+  __syncthreads();
+
+  int it = 0;
+  bool stop = false, dead = false;
+  while (it < a.niter && !stop) {
+    const int buf = it & 1;
+    unsigned long long *slot = a.slots + 2ull * G * kHogCopies * buf;
+    const unsigned long long mark = (unsigned long long)((it >> 1) & 1) << 63;
+    if (warp == 0) {
+      // This CTA's best pixel; its segments lie in the image's order.
+      unsigned long long bv = 0;
+      int bi = kNoPixel;
+      for (int i = lane; i < mine; i += 32)
+        if (s_segi[i] != kNone) hog_take(s_segv[i], i, &bv, &bi);
+      int leader = hog_best_lane(bv, (unsigned)bi);
+      unsigned long long w1 = 0;
+      if (lane == leader) {
+        unsigned word = 0x80000000u;  // bit 31: no pixel, bit 30: the residual is in lookup, bit 29: it is negative
+        if (bi != kNoPixel) {
+          const int p = s_segi[bi];
+          double r;
+          if (SMEM) {
+            r = s_res[bi * kHogSeg + p];
+          } else {
+            long long col;
+            const long long row = seg_row(bi, &col);
+            r = a.res[row * a.ny + col + p];
+          }
+          const unsigned long long rb = (unsigned long long)__double_as_longlong(r);
+          word = (unsigned)p;  // below 2^29
+          if ((rb & kAbsMask) != bv) {
+            word |= 0x40000000u;
+            *(volatile double *)&a.lookup[(size_t)buf * G + cta] = r;
+            __threadfence();
+          } else if (rb >> 63) {
+            word |= 0x20000000u;
+          }
+        }
+        // word 0: value, mark; word 1: generation (8 bits; the slot's last one is it - 2), segment (24), word (32)
+        w1 = (unsigned long long)((unsigned)(it & 0xff) << 24 | ((unsigned)bi & 0xffffffu)) << 32 | word;
+      }
+      bv = __shfl_sync(0xffffffffu, bv, leader);
+      w1 = __shfl_sync(0xffffffffu, w1, leader);
+      if (lane < kHogCopies) hog_put(slot + 2 * ((size_t)lane * G + cta), bv | mark, w1);
+      // Everybody's best pixel, kHogPoll slots a lane, all loads of a round in flight together; the key (segment,
+      // pixel in it) orders pixels as the image does.
+      const unsigned long long *from = slot + 2 * (size_t)(cta % kHogCopies) * G;
+      unsigned long long v = 0, key = ~0ull, w0[kHogPoll], w2[kHogPoll];
+      unsigned word = 0x80000000u, todo = 0;
+#pragma unroll
+      for (int k = 0; k < kHogPoll; ++k) todo |= (lane + 32 * k < G ? 1u : 0u) << k;
+      for (int tries = 0; __any_sync(0xffffffffu, todo) && tries < kHogTries; ++tries) {
+#pragma unroll
+        for (int k = 0; k < kHogPoll; ++k)
+          if ((todo >> k) & 1) hog_get(from + 2 * (lane + 32 * k), &w0[k], &w2[k]);
+#pragma unroll
+        for (int k = 0; k < kHogPoll; ++k)
+          if (((todo >> k) & 1) && (w0[k] & ~kAbsMask) == mark && (unsigned)(w2[k] >> 56) == (unsigned)(it & 0xff)) {
+            todo &= ~(1u << k);
+            const unsigned long long t = w0[k] & kAbsMask;
+            const unsigned long long at =
+                (unsigned long long)(lane + 32 * k + ((unsigned)(w2[k] >> 32) & 0xffffffu) * G) << 32 |
+                ((unsigned)w2[k] & 0x1fffffffu);
+            if (!((unsigned)w2[k] >> 31) && (t > v || (t == v && at < key))) {
+              v = t;
+              key = at;
+              word = (unsigned)w2[k];
+            }
+          }
+      }
+      const bool late = __any_sync(0xffffffffu, todo);
+      leader = hog_best_lane(v, key);
+      if (lane == leader) {
+        s_bits = v;
+        s_key = key;
+        s_word = word;
+        s_end = late ? 2 : (int)(word >> 31);  // 1: no pixel qualifies
+      }
+    }
+    __syncthreads();
+    if (s_end) {
+      dead = s_end == 2;
+      break;
+    }
+    const unsigned long long key = s_key;
+    const unsigned seg = (unsigned)(key >> 32);
+    const unsigned mrow = seg_div(seg);
+    const long long mx = mrow, my = (long long)(seg - mrow * spr) * width + (unsigned)key;
+    if (threadIdx.x == 0) {
+      const unsigned word = s_word;
+      double r = __longlong_as_double((long long)(s_bits | ((unsigned long long)((word >> 29) & 1) << 63)));
+      if ((word >> 30) & 1) {
+        __threadfence();
+        r = *(volatile double *)&a.lookup[(size_t)buf * G + seg % G];
+      }
+      s_mval = hog_quotient(__dmul_rn(r, a.gain), a.pmax, rcp);
+    }
+    // The patch (overlapIndices of the reference): rows [r0, r1), columns [c0, c1), PSF pixel (x - mx + wx, y - my + wy).
+    const long long r0 = max(0ll, mx - wx), r1 = min(a.nx, mx + wx);
+    const long long c0 = max(0ll, my - wy), c1 = min(my + wy, a.ny);
+    const int first = (int)r0 * (int)spr - cta, last = (int)r1 * (int)spr - cta;  // i G in [first, last)
+    const int i0 = first > 0 ? (int)((unsigned)(first + G - 1) / G) : 0;
+    const int i1 = last > 0 ? (int)((unsigned)(last + G - 1) / G) : 0;
+    const int start = i0 + warp;
+    double pre[kHogPx];
+    if (SMEM && start < i1) {  // the first segment's PSF values come in while thread 0 divides
+      long long col;
+      const long long row = seg_row(start, &col);
+      const double *prow = a.psf + (row - mx + wx) * a.pny + (wy - my);
+#pragma unroll
+      for (int j = 0; j < kHogPx; ++j) {
+        const long long c = col + lane + 32 * j;
+        pre[j] = c >= c0 && c < c1 ? prow[c] : 0.0;
+      }
+    }
+    __syncthreads();
+    const double mval = s_mval;
+    if (threadIdx.x == kHogThreads - 1) {
+      // the last warp, which has a segment least often: the component, and the stopping test on the updated peak
+      const unsigned word = s_word;
+      double r = __longlong_as_double((long long)(s_bits | ((unsigned long long)((word >> 29) & 1) << 63)));
+      if ((word >> 30) & 1) r = *(volatile double *)&a.lookup[(size_t)buf * G + seg % G];
+      s_stop = fabs(__dsub_rn(r, __dmul_rn(centre, mval))) < a.stop_level;
+      if (seg % G == (unsigned)cta) a.comps[mx * a.ny + my] = __dadd_rn(a.comps[mx * a.ny + my], mval);
+    }
+    for (int i = start; i < i1; i += kHogThreads / 32) {
+      long long col;
+      const long long row = seg_row(i, &col);
+      if (col >= c1 || col + width <= c0) continue;
+      scan(i, row, col, a.psf + (row - mx + wx) * a.pny + (wy - my), c0, c1, mval, SMEM && i == start ? pre : nullptr);
+    }
+    ++it;
+    __syncthreads();
+    stop = s_stop;
+  }
+  if (SMEM)
+    for (int i = warp; i < mine; i += kHogThreads / 32) {
+      long long col;
+      const long long row = seg_row(i, &col);
+      for (int p = lane; p < kHogSeg && col + p < a.ny; p += 32) a.res[row * a.ny + col + p] = s_res[i * kHogSeg + p];
+    }
+  if (cta == 0 && threadIdx.x == 0) {
+    a.status->iters = it;
+    a.status->stop = stop || it < a.niter;
+  }
+  if (dead && threadIdx.x == 0) a.status->error = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -577,51 +833,78 @@ extern "C" int arlgpu_hogbom(const double *dirty, const double *psf, const doubl
   if (!(psf_max > 0.0)) return fail(ARLGPU_ERR_INVALID, "psf maximum must be > 0");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const long long n = (long long)nx * ny;
-  const int fblocks = nblk(n, 152 * 4);
-  const int sblocks = nblk((long long)psf_nx * psf_ny, 152 * 8);
-  HogState *state = nullptr;
-  Best *partial = nullptr;
-  ARL_CUDA(cudaMallocAsync(&state, sizeof(HogState), st));
-  int rc = ARLGPU_OK;
-  if (cudaMallocAsync(&partial, sizeof(Best) * fblocks, st) != cudaSuccess) {
-    cudaFreeAsync(state, st);
-    return fail(ARLGPU_ERR_CUDA, "cudaMallocAsync failed");
-  }
   const double absthresh = fmax(thresh, fracthresh * dirty_absmax);
-  const double stop_level = 0.9 * absthresh;
-  constexpr int kCheck = 64;
-  int it = 0;
-  HogState hs{};
-  do {
-    if (cudaMemsetAsync(state, 0, sizeof(HogState), st) != cudaSuccess ||
-        cudaMemcpyAsync(res, dirty, sizeof(double) * n, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemsetAsync(comps, 0, sizeof(double) * n, st) != cudaSuccess) {
-      rc = fail(ARLGPU_ERR_CUDA, "hogbom set-up failed");
+  HogArgs args{};
+  args.psf = psf;
+  args.window = window;
+  args.comps = comps;
+  args.res = res;
+  args.nx = nx;
+  args.ny = ny;
+  args.pnx = psf_nx;
+  args.pny = psf_ny;
+  args.gain = gain;
+  args.pmax = psf_max;
+  args.stop_level = 0.9 * absthresh;
+  int dev = 0, sms = 0, smem_max = 0;
+  ARL_CUDA(cudaGetDevice(&dev));
+  ARL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  ARL_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  const long long odd = std::min((sms - 1) | 1, 32 * kHogPoll - 1);
+  // The residual in shared memory where it fits, in 256-pixel segments; else in
+  // global memory, in segments wide enough for 8192 to serve a CTA.
+  auto segments = [&](long long width) { return (long long)nx * ((ny + width - 1) / width); };
+  long long width = kHogSeg, ctas = std::min(odd, segments(width));
+  long long nloc = (segments(width) + ctas - 1) / ctas;
+  const size_t statics = 1024;  // at least the kernel's static shared memory
+  size_t smem = (size_t)nloc * (kHogSeg * 8 + 64 + 10);
+  const bool in_smem = smem + statics <= (size_t)smem_max;
+  if (!in_smem) {
+    while ((segments(width) + odd - 1) / odd > 8192 && width < ny) width <<= 1;
+    ctas = std::min(odd, segments(width));
+    nloc = (segments(width) + ctas - 1) / ctas;
+    smem = (size_t)nloc * 12;
+    if (smem + statics > (size_t)smem_max) smem = 0;  // a tall, narrow image: the bests in global memory
+  }
+  args.width = (int)width;
+  args.nloc = (int)nloc;
+  const void *kern = in_smem ? (const void *)k_hogbom<true> : (const void *)k_hogbom<false>;
+  ARL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - (int)statics));
+  // status, then the slots and the lookup values
+  const size_t slot_bytes = (size_t)ctas * kHogCopies * 2 * 2 * sizeof(unsigned long long);
+  const size_t bests = smem ? 0 : (size_t)ctas * nloc * 16;
+  const size_t bytes = 16 + slot_bytes + (size_t)ctas * 2 * sizeof(double) + bests;
+  char *ws = nullptr;
+  ARL_CUDA(cudaMallocAsync(&ws, bytes, st));
+  args.status = reinterpret_cast<HogStatus *>(ws);
+  args.slots = reinterpret_cast<unsigned long long *>(ws + 16);
+  args.lookup = reinterpret_cast<double *>(ws + 16 + slot_bytes);
+  args.bests = bests ? reinterpret_cast<unsigned char *>(args.lookup + 2 * ctas) : nullptr;
+  int rc = ARLGPU_OK, done = 0;
+  HogStatus hs{};
+  if (cudaMemsetAsync(comps, 0, sizeof(double) * n, st) != cudaSuccess) rc = fail(ARLGPU_ERR_CUDA, "hogbom set-up failed");
+  args.src = dirty;
+  constexpr int kBatch = 20000;  // iterations per launch: some tens of milliseconds
+  while (rc == ARLGPU_OK && done < niter && !hs.stop) {
+    args.niter = std::min(niter - done, kBatch);
+    void *params[] = {&args};
+    if (cudaMemsetAsync(args.status, 0, sizeof(HogStatus), st) != cudaSuccess ||
+        cudaMemsetAsync(args.slots, 0xff, slot_bytes, st) != cudaSuccess ||
+        cudaLaunchCooperativeKernel(kern, dim3((unsigned)ctas), dim3(kHogThreads), params, smem, st) != cudaSuccess) {
+      rc = fail(ARLGPU_ERR_CUDA, "hogbom launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       break;
     }
-    while (it < niter) {
-      const int batch = niter - it < kCheck ? niter - it : kCheck;
-      for (int k = 0; k < batch; ++k) {
-        k_hog_find<<<fblocks, kFindThreads, 0, st>>>(res, window, n, gain, psf_max, comps, partial, state);
-        k_hog_sub<<<sblocks, 256, 0, st>>>(res, nx, ny, psf, psf_nx, psf_ny, stop_level, state);
-      }
-      count_launch(2 * batch);
-      it += batch;
-      if (cudaGetLastError() != cudaSuccess) {
-        rc = fail(ARLGPU_ERR_CUDA, "hogbom launch failed");
-        break;
-      }
-      if (cudaMemcpyAsync(&hs, state, sizeof hs, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess) {
-        rc = fail(ARLGPU_ERR_CUDA, "hogbom state read failed");
-        break;
-      }
-      if (hs.stop) break;
-    }
-  } while (false);
-  *iterations = hs.iters;
-  cudaFreeAsync(partial, st);
-  cudaFreeAsync(state, st);
+    count_launch(1);
+    if (cudaMemcpyAsync(&hs, args.status, sizeof hs, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      rc = fail(ARLGPU_ERR_CUDA, "hogbom state read failed");
+    else if (hs.error)
+      rc = fail(ARLGPU_ERR_CUDA, "hogbom: a CTA waited too long for the others");
+    done += hs.iters;
+    args.src = res;
+  }
+  *iterations = done;
+  cudaFreeAsync(ws, st);
   return rc;
 }
 
