@@ -106,7 +106,7 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
 
 // Workspace carve-up for a plan over nvis rows.
 struct PlanBufs {
-  uint32_t *keys;
+  uint32_t *keys;     // rank of each row within its bin
   RowMap *maps;
   uint32_t *sidx;
   RowMap *smap;

@@ -228,16 +228,19 @@ __device__ __forceinline__ bool fix_round(double x, const arlgpu_axis &a, double
   return true;
 }
 
-// Nearest-plane index of one axis in [0, n), or -1 outside: the fixed-point
-// decision, and NumPy's exact sequence for that axis alone where the value
-// lies within the tolerance of a half-integer.  Whole sets of rows can sit on
-// such a tie: with an even number of w slices centred on w = 0, every row of
-// a coplanar array at transit (w = 0 up to rounding) does.
-__device__ __forceinline__ int plane_index(double x, const arlgpu_axis &a, double rcp, int tq, int n, bool fixint,
-                                           const FixAxis &fa) {
-  int idx;
-  if (fixint ? int_round(x, fa, tq + kFixSlack, &idx) : fix_round(x, a, rcp, tq, &idx))
-    return idx >= 0 && idx < n ? idx : -1;
+// Nearest-plane index of one axis in [0, n), or -1 outside, by the fixed-point
+// decision; false where the value lies within the tolerance of a half-integer.
+__device__ __forceinline__ bool plane_index(double x, const arlgpu_axis &a, double rcp, int tq, int n, bool fixint,
+                                            const FixAxis &fa, int *idx) {
+  if (!(fixint ? int_round(x, fa, tq + kFixSlack, idx) : fix_round(x, a, rcp, tq, idx))) return false;
+  if (*idx < 0 || *idx >= n) *idx = -1;
+  return true;
+}
+
+// The same by NumPy's exact sequence.  Whole sets of rows can sit on a tie: with an
+// even number of w slices centred on w = 0, every row of a coplanar array at
+// transit (w = 0 up to rounding) does.  So such rows do only this axis again.
+__device__ __forceinline__ int plane_index_exact(double x, const arlgpu_axis &a, int n) {
   const double p = rint(w2p_exact(x, a));  // range test in double: no wrap when narrowed
   return p >= 0.0 && p < (double)n ? (int)p : -1;
 }
@@ -257,33 +260,20 @@ __device__ __forceinline__ bool map_fixed(double u, double v, double w, double f
                fix_axis_x(v, g.rOv, g.cOv, g.tq_v, g.O, g.log2O, pv, vf))) {
     return false;
   }
-  *zg = g.skip_zg ? 0 : plane_index(w, g.gw, g.rcp_gw, g.tq_w, g.nw, g.fixint, g.fw);
-  *zc = g.skip_zc ? 0 : plane_index(w, g.cz, g.rcp_cz, g.tq_z, g.nz, g.fixint, g.fz);
-  *ch = plane_index(f, g.gf, g.rcp_gf, g.tq_f, min(g.nchan, g.cf_nchan), g.fixint, g.ff);
+  *zg = *zc = 0;
+  if (!g.skip_zg && !plane_index(w, g.gw, g.rcp_gw, g.tq_w, g.nw, g.fixint, g.fw, zg))
+    *zg = plane_index_exact(w, g.gw, g.nw);
+  if (!g.skip_zc && !plane_index(w, g.cz, g.rcp_cz, g.tq_z, g.nz, g.fixint, g.fz, zc))
+    *zc = plane_index_exact(w, g.cz, g.nz);
+  if (!plane_index(f, g.gf, g.rcp_gf, g.tq_f, min(g.nchan, g.cf_nchan), g.fixint, g.ff, ch))
+    *ch = plane_index_exact(f, g.gf, min(g.nchan, g.cf_nchan));
   return true;
 }
 
-__device__ __forceinline__ Mapped map_row(double u, double v, double w, double f, const Geom &g) {
+// The rest of a row's mapping: the window of its plane's support inside the grid.
+__device__ __forceinline__ Mapped map_finish(bool ok, int pu, int pv, int uf, int vf, int zg, int zc, int ch,
+                                             const Geom &g) {
   Mapped m;
-  bool ok;
-  int pu, pv, uf, vf, zg, zc, ch;
-  if (map_fixed(u, v, w, f, g, &pu, &pv, &uf, &vf, &zg, &zc, &ch)) {
-    // uf, vf lie in [0, O) by construction
-    ok = pu >= 0 && pu < g.nx && pv >= 0 && pv < g.ny && zg >= 0 && zc >= 0 && ch >= 0;
-  } else {
-    const RawMap r = map_raw(u, v, w, f, g);
-    // Range checks in double so huge values cannot wrap when narrowed.
-    ok = r.pu >= 0.0 && r.pu < g.nx && r.pv >= 0.0 && r.pv < g.ny && r.uf >= 0.0 && r.uf < g.O && r.vf >= 0.0 &&
-         r.vf < g.O && r.zg >= 0.0 && r.zg < g.nw && r.zc >= 0.0 && r.zc < g.nz && r.ch >= 0.0 && r.ch < g.nchan &&
-         r.ch < g.cf_nchan;
-    pu = ok ? (int32_t)r.pu : 0;
-    pv = ok ? (int32_t)r.pv : 0;
-    uf = ok ? (int32_t)r.uf : 0;
-    vf = ok ? (int32_t)r.vf : 0;
-    zg = ok ? (int32_t)r.zg : 0;
-    zc = ok ? (int32_t)r.zc : 0;
-    ch = ok ? (int32_t)r.ch : 0;
-  }
   m.pu = ok ? pu : -1;
   m.pv = ok ? pv : -1;
   m.uf = ok ? uf : 0;
@@ -297,6 +287,31 @@ __device__ __forceinline__ Mapped map_row(double u, double v, double w, double f
   }
   m.ok = ok;
   return m;
+}
+
+// One row by the fixed-point decisions alone; false where they do not hold.
+__device__ __forceinline__ bool map_row_fixed(double u, double v, double w, double f, const Geom &g, Mapped *m) {
+  int pu, pv, uf, vf, zg, zc, ch;
+  if (!map_fixed(u, v, w, f, g, &pu, &pv, &uf, &vf, &zg, &zc, &ch)) return false;
+  // uf, vf lie in [0, O) by construction
+  *m = map_finish(pu >= 0 && pu < g.nx && pv >= 0 && pv < g.ny && zg >= 0 && zc >= 0 && ch >= 0, pu, pv, uf, vf, zg, zc,
+                  ch, g);
+  return true;
+}
+
+__device__ __forceinline__ Mapped map_row_exact(double u, double v, double w, double f, const Geom &g) {
+  const RawMap r = map_raw(u, v, w, f, g);
+  // Range checks in double so huge values cannot wrap when narrowed.
+  const bool ok = r.pu >= 0.0 && r.pu < g.nx && r.pv >= 0.0 && r.pv < g.ny && r.uf >= 0.0 && r.uf < g.O &&
+                  r.vf >= 0.0 && r.vf < g.O && r.zg >= 0.0 && r.zg < g.nw && r.zc >= 0.0 && r.zc < g.nz &&
+                  r.ch >= 0.0 && r.ch < g.nchan && r.ch < g.cf_nchan;
+  return map_finish(ok, ok ? (int32_t)r.pu : 0, ok ? (int32_t)r.pv : 0, ok ? (int32_t)r.uf : 0, ok ? (int32_t)r.vf : 0,
+                    ok ? (int32_t)r.zg : 0, ok ? (int32_t)r.zc : 0, ok ? (int32_t)r.ch : 0, g);
+}
+
+__device__ __forceinline__ Mapped map_row(double u, double v, double w, double f, const Geom &g) {
+  Mapped m;
+  return map_row_fixed(u, v, w, f, g, &m) ? m : map_row_exact(u, v, w, f, g);
 }
 
 __device__ __forceinline__ uint32_t bin_of(int ch, int zg, int pu, int pv, const Geom &g) {
