@@ -16,6 +16,7 @@
 // one channel map), gives the gradient of a DFT-predicted chi^2 with respect
 // to the component fluxes; the gradient checks use it as a dense reference.
 #include "common.cuh"
+#include "dsmath.cuh"
 
 namespace arlgpu {
 
@@ -123,25 +124,11 @@ __device__ __forceinline__ bool fix_words(double x, int scale, int *hi, int *lo)
   return s >= 0 && *hi != (int)0x80000000;  // the words' range, also after rounding hi
 }
 
-// cos and sin of 2 pi t, t = phase 2^-32 turns: y = the offset from the
-// quadrant's centre in eighths of a turn, |y| <= 1.  Least-maximum fits of
-// sin(pi y / 4) / y (degree 3 in y^2, 2.4e-9) and cos(pi y / 4) (degree 4,
-// 5e-11); pi / 4 is split so that its rounding does not scale the sine.
+// cos and sin of 2 pi t, t = phase 2^-32 turns.
 __device__ __forceinline__ void sincos_fix(int phase, float *c, float *s) {
   const unsigned q = ((unsigned)phase + 0x20000000u) >> 30;
   const float y = (float)(int)((unsigned)phase - (q << 30)) * 1.862645149230957e-9f;  // 2^-29
-  const float z = y * y;
-  float a = fmaf(z, -3.59545078e-05f, 2.49000713e-03f);
-  a = fmaf(a, z, -8.07454348e-02f);
-  a = fmaf(a, z, -2.4e-08f);  // pi / 4 = 0.78539818525 - 2.19e-8, less the fit's -2.1e-9
-  const float sn = fmaf(y, 0.78539818525f, y * a);
-  float b = fmaf(z, 3.52981134e-06f, -3.25938614e-04f);
-  b = fmaf(b, z, 1.58543252e-02f);
-  b = fmaf(b, z, -3.08425135e-01f);
-  const float cs = fmaf(b, z, 1.f);
-  const float cc = (q & 1) ? sn : cs, ss = (q & 1) ? cs : sn;
-  *c = __int_as_float(__float_as_int(cc) ^ (((q + 1) & 2) << 30));
-  *s = __int_as_float(__float_as_int(ss) ^ ((q & 2) << 30));
+  sincos_quadrant(y, q, c, s);
 }
 
 template <int NPOL, int RPT>

@@ -10,24 +10,35 @@
 // (~6e4 at the edge of a PSWF-corrected field), so the inverse transform must
 // be much more accurate than FP32.  GB300 runs FP64 at 1/64 of its FP32 rate,
 // which makes cuFFT's FP64 transform of an 8192^2 plane compute-bound at
-// ~14 ms.  Here every complex value is a pair of double-single numbers
-// (float4: re.hi, re.lo, im.hi, im.lo; ~48-bit significands) and all
-// arithmetic runs on the FP32 pipes.
+// ~14 ms.  Here every complex value is a pair of double-single numbers (~48-bit
+// significands) and all arithmetic runs on the FP32 pipes.
 //
-// Layout: a plane of ny x nx points, row-major.  Three passes per plane:
+// Layout: a plane of ny x nx points, row-major, a point as float4 (re.hi, im.hi,
+// re.lo, im.lo).  Three passes per plane:
 //   rows   one CTA per 4096 points (4096 / nx rows, or half of an
 //          8192-point row): FP32 grid (w-planes summed, chk sign) -> row
-//          DFTs in shared memory -> DS buffer
-//   cols1  ny = N1 * N2: DFTs of length N1 over rows n2 + N2 n1 of 32 or 64
+//          DFTs -> DS buffer
+//   cols1  ny = N1 * N2: DFTs of length N1 over rows n2 + N2 n1 of 32 or more
 //          adjacent columns, times exp(2 pi i n2 k1 / ny), in place
 //   cols2  DFTs of length N2 over rows N2 k1 + n2 -> row k1 + N1 k2, with the
 //          epilogue fused: image write (invert_2d) or the w-screen product
 //          summed over the slices of the group (w-stacking)
-// Each DFT is a Stockham radix-4 (one radix-2 pass for odd log2) sequence in
-// shared memory: the first pass reads global memory, the last writes the
-// epilogue, both coalesced.  Twiddles come from one DS table of
-// exp(2 pi i m / 16384) computed once per device in FP64.
+// What bounds them is the FP32 pipe, about 790 operations a point of 8192^2 (1.4 ms a
+// plane) against 4.5 GB of traffic (0.7 ms), so the passes spend their issue slots
+// on those operations:
+//   * a thread transforms 16 points in registers (radix 16, or 16 / R of radix R), so
+//     that a DFT of up to 4096 points crosses shared memory twice and one of up to
+//     128 once; the lengths are compile-time constants, and the first pass reads
+//     global memory into registers (16 loads in flight), the last writes the
+//     epilogue;
+//   * real and imaginary parts are adjacent, so that sums are packed FP32 pairs:
+//     the same lane rate as single ones, for half the issue slots.
+// Radix-4 passes of run-time length, one butterfly a thread through shared
+// memory, were at 3.15 ms a plane of 8192^2 (w-stack, 32 planes: rows 1.20, cols1
+// 0.74, cols2 1.20 ms); now 1.92 ms (0.62, 0.56, 0.73).
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "dsmath.cuh"
@@ -38,21 +49,30 @@ void count_launch(unsigned n);
 
 constexpr int kLog2Tw = 14;
 constexpr int kTw = 1 << kLog2Tw;
-__device__ float4 g_tw[kTw];  // exp(+2 pi i m / 16384): (cos hi, cos lo, sin hi, sin lo)
+// exp(+2 pi i m / 16384) as (cos hi, sin hi, cos lo, sin lo), for the twiddles between the column passes
+__device__ float4 g_tw[kTw];
+// exp(+2 pi i m k / (16 M)) at [k][m], for the passes with M points left: the lanes of a warp take adjacent m
+__device__ float4 g_tw256[16 * 256];
+__device__ float4 g_tw16[16 * 16];
 
 __global__ void k_tw_init() {
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < kTw; m += gridDim.x * blockDim.x) {
+  auto at = [](int m, int n) {  // exp(2 pi i m / n)
     double s, c;
-    sincospi((double)m / (double)(kTw / 2), &s, &c);
+    sincospi(2.0 * (double)(m % n) / (double)n, &s, &c);
     const dsf cc = ds_from_double(c), ss = ds_from_double(s);
-    g_tw[m] = make_float4(cc.hi, cc.lo, ss.hi, ss.lo);
+    return make_float4(cc.hi, ss.hi, cc.lo, ss.lo);
+  };
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kTw; i += gridDim.x * blockDim.x) {
+    g_tw[i] = at(i, kTw);
+    if (i < 16 * 256) g_tw256[i] = at((i >> 8) * (i & 255), 4096);
+    if (i < 16 * 16) g_tw16[i] = at((i >> 4) * (i & 15), 256);
   }
 }
 
 static std::atomic<unsigned> g_tw_ready{0};
 
-// The table is filled once per device on a stream that is not capturing
-// (synchronised so that every later stream sees it); under capture the fill
+// The tables are filled once per device on a stream that is not capturing
+// (synchronised so that every later stream sees them); under capture the fill
 // is recorded into the graph instead, every time, so a graph never relies on
 // a fill that did not run.
 static int ensure_twiddles(cudaStream_t st) {
@@ -60,7 +80,7 @@ static int ensure_twiddles(cudaStream_t st) {
   ARL_CUDA(cudaGetDevice(&dev));
   const unsigned bit = 1u << (dev & 31);
   if (g_tw_ready.load() & bit) return ARLGPU_OK;
-  k_tw_init<<<16, 256, 0, st>>>();
+  k_tw_init<<<64, 256, 0, st>>>();
   ARL_LAUNCH_CHECK();
   count_launch(1);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -73,333 +93,369 @@ static int ensure_twiddles(cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Complex double-single arithmetic on float4 (re.hi, re.lo, im.hi, im.lo).
+// Packed FP32 pairs and complex double-single values.  h = (re.hi, im.hi), l = the
+// low parts.  Sums are left unnormalised (hi + lo still equals the value; the
+// next error-free sum or twiddle product absorbs it), which NumPy float32 emulation
+// shows costs nothing measurable (7.9e-15 against 7.4e-15 of the scale at 8192 points).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float4 c_add_nr(float4 a, float4 b) {  // unnormalised sum
-  const dsf r = two_sum(a.x, b.x), i = two_sum(a.z, b.z);
-  return make_float4(r.hi, __fadd_rn(r.lo, __fadd_rn(a.y, b.y)), i.hi, __fadd_rn(i.lo, __fadd_rn(a.w, b.w)));
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
 }
-__device__ __forceinline__ float4 c_neg(float4 a) { return make_float4(-a.x, -a.y, -a.z, -a.w); }
-__device__ __forceinline__ float4 c_norm(float4 a) {
-  const dsf r = quick_two_sum(a.x, a.y), i = quick_two_sum(a.z, a.w);
-  return make_float4(r.hi, r.lo, i.hi, i.lo);
+__device__ __forceinline__ float2 un(f2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
 }
-// i * a
-__device__ __forceinline__ float4 c_muli(float4 a) { return make_float4(-a.z, -a.w, a.x, a.y); }
-
-// a * w (w a unit twiddle).
-__device__ __forceinline__ float4 c_mul(float4 a, float4 w) {
-  const dsf p1 = two_prod(a.x, w.x), p2 = two_prod(a.z, w.z);
-  const dsf s1 = two_sum(p1.hi, -p2.hi);
-  float e1 = __fadd_rn(s1.lo, __fsub_rn(p1.lo, p2.lo));
-  e1 = __fmaf_rn(a.x, w.y, e1);
-  e1 = __fmaf_rn(a.y, w.x, e1);
-  e1 = __fmaf_rn(-a.z, w.w, e1);
-  e1 = __fmaf_rn(-a.w, w.z, e1);
-  const dsf p3 = two_prod(a.x, w.z), p4 = two_prod(a.z, w.x);
-  const dsf s2 = two_sum(p3.hi, p4.hi);
-  float e2 = __fadd_rn(s2.lo, __fadd_rn(p3.lo, p4.lo));
-  e2 = __fmaf_rn(a.x, w.w, e2);
-  e2 = __fmaf_rn(a.y, w.z, e2);
-  e2 = __fmaf_rn(a.z, w.y, e2);
-  e2 = __fmaf_rn(a.w, w.x, e2);
-  const dsf r = quick_two_sum(s1.hi, e1), i = quick_two_sum(s2.hi, e2);
-  return make_float4(r.hi, r.lo, i.hi, i.lo);
+__device__ __forceinline__ f2 swp(f2 a) {
+  const float2 v = un(a);
+  return pk(v.y, v.x);
 }
-
-// exp(+2 pi i m / 2^log2n) for 0 <= m < 2^log2n <= 16384
-__device__ __forceinline__ float4 twiddle(int m, int log2n) { return __ldg(&g_tw[m << (kLog2Tw - log2n)]); }
-
-// 16-byte global -> shared copies that bypass the registers, all in flight
-// before one wait (the column passes stage their 64 KiB tiles this way).
-__device__ __forceinline__ void cp_async16(float4 *smem, const float4 *gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
-// ---------------------------------------------------------------------------
-// In-place radix-2^2 decimation-in-frequency transform (inverse sign) of
-// S = 2^log2S sequences of L = 2^log2L points held in shared memory at
-// pos(n, q): natural order in, bit-reversed order out.  Each butterfly reads
-// and writes the same four slots, so a thread holds one butterfly at a time
-// and a pass needs one barrier.  Two radix-2 stages of spans h and h/2 fuse
-// into one butterfly on the points n0 + {0, h/2, h, 3h/2} of a block of 2h:
-//   a = x0 + x2, b = x0 - x2, c = x1 + x3, d = i (x1 - x3), w = exp(2 pi i j / 2h)
-//   y0 = a + c, y1 = (a - c) w^2, y2 = (b + d) w, y3 = (b - d) w^3
-// and an odd log2 L ends with one radix-2 stage of span 1.  Sums are left
-// unnormalised (hi + lo still equals the value; the next error-free sum or
-// twiddle product absorbs it), which NumPy float32 emulation shows costs
-// nothing measurable (7.9e-15 against 7.4e-15 of the scale at 8192 points).
-// tw(m, lw) = exp(2 pi i m / 2^lw).
-// ---------------------------------------------------------------------------
-template <int T, typename Pos, typename Tw>
-__device__ __forceinline__ void ds_dif_cta(float4 *sm, int log2L, int log2S, bool seqfast, Pos pos, Tw tw) {
-  const int S1 = (1 << log2S) - 1;
-  const int nb4 = 1 << (log2L - 2 + log2S);
-  int log2h = log2L - 1;
-  for (; log2h >= 1; log2h -= 2) {
-    const int lq = log2h - 1, J1 = (1 << lq) - 1;
-    const int lblk = log2L - log2h - 1;  // log2 of the blocks per sequence
-    for (int bb = threadIdx.x; bb < nb4; bb += T) {
-      int q, jp, blk;
-      if (seqfast) {
-        q = bb & S1;
-        const int rest = bb >> log2S;
-        jp = rest & J1;
-        blk = rest >> lq;
-      } else {
-        jp = bb & J1;
-        const int rest = bb >> lq;
-        blk = rest & ((1 << lblk) - 1);
-        q = rest >> lblk;
-      }
-      const int n0 = (blk << (log2h + 1)) + jp, hh = 1 << lq;
-      const int i0 = pos(n0, q), i1 = pos(n0 + hh, q), i2 = pos(n0 + 2 * hh, q), i3 = pos(n0 + 3 * hh, q);
-      const float4 x0 = sm[i0], x1 = sm[i1], x2 = sm[i2], x3 = sm[i3];
-      const float4 a = c_add_nr(x0, x2), b = c_add_nr(x0, c_neg(x2));
-      const float4 c = c_add_nr(x1, x3), d = c_muli(c_add_nr(x1, c_neg(x3)));
-      float4 y1 = c_add_nr(a, c_neg(c)), y2 = c_add_nr(b, d), y3 = c_add_nr(b, c_neg(d));
-      if (jp) {
-        const int lw = log2h + 1;
-        y2 = c_mul(y2, tw(jp, lw));
-        y1 = c_mul(y1, tw(2 * jp, lw));
-        y3 = c_mul(y3, tw(3 * jp, lw));
-      }
-      sm[i0] = c_add_nr(a, c);
-      sm[i1] = y1;
-      sm[i2] = y2;
-      sm[i3] = y3;
-    }
-    __syncthreads();
-  }
-  if (log2h == 0) {
-    const int nb2 = 1 << (log2L - 1 + log2S), lb = log2L - 1, B1 = (1 << lb) - 1;
-    for (int bb = threadIdx.x; bb < nb2; bb += T) {
-      const int q = seqfast ? (bb & S1) : (bb >> lb), i = seqfast ? (bb >> log2S) : (bb & B1);
-      const int i0 = pos(2 * i, q), i1 = pos(2 * i + 1, q);
-      const float4 x0 = sm[i0], x1 = sm[i1];
-      sm[i0] = c_add_nr(x0, x1);
-      sm[i1] = c_add_nr(x0, c_neg(x1));
-    }
-    __syncthreads();
-  }
-}
-
-// Global table lookup, for the row transforms.
-struct TwGlobal {
-  __device__ __forceinline__ float4 operator()(int m, int lw) const { return twiddle(m, lw); }
+struct cds {
+  f2 h, l;
 };
-// exp(2 pi i m / L) for m < L <= 128 staged in shared memory by the column
-// kernels (the only twiddles their transforms use).
-struct TwShared {
-  const float4 *t;
-  int log2L;
-  __device__ __forceinline__ float4 operator()(int m, int lw) const { return t[m << (log2L - lw)]; }
-};
-__device__ __forceinline__ void stage_twiddles(float4 *t, int log2L) {
-  for (int m = threadIdx.x; m < (1 << log2L); m += blockDim.x) t[m] = twiddle(m, log2L);
+__device__ __forceinline__ cds c_from(float4 v) { return {pk(v.x, v.y), pk(v.z, v.w)}; }
+__device__ __forceinline__ float4 c_to(cds a) {
+  const float2 h = un(a.h), l = un(a.l);
+  return make_float4(h.x, h.y, l.x, l.y);
 }
 
-__device__ __forceinline__ int brev(int k, int log2L) { return (int)(__brev((unsigned)k) >> (32 - log2L)); }
+// a + b, a - b: error-free sums of the high parts, low parts and errors added.
+__device__ __forceinline__ cds c_add(cds a, cds b) {
+  const f2 s = add2(a.h, b.h), v = sub2(s, a.h), e = add2(sub2(a.h, sub2(s, v)), sub2(b.h, v));
+  return {s, add2(e, add2(a.l, b.l))};
+}
+__device__ __forceinline__ cds c_sub(cds a, cds b) {
+  const f2 s = sub2(a.h, b.h), v = sub2(s, a.h), e = sub2(sub2(a.h, sub2(s, v)), add2(b.h, v));
+  return {s, add2(e, sub2(a.l, b.l))};
+}
+// a + i b (SIGN > 0) or a - i b: b's parts change places, and products with +-1 in the fused operations (exact) give
+// their signs.
+template <int SIGN>
+__device__ __forceinline__ cds c_addi(cds a, cds b) {
+  const f2 j = SIGN > 0 ? pk(-1.f, 1.f) : pk(1.f, -1.f);
+  const f2 bh = swp(b.h), s = fma2(bh, j, a.h), v = sub2(a.h, s);  // v = -(s - a)
+  const f2 e = add2(sub2(a.h, add2(s, v)), fma2(bh, j, v));
+  return {s, add2(e, fma2(swp(b.l), j, a.l))};
+}
+
+// a * w: the four products error-free through FMAs, part by part (their operands need no re-pairing), the rest packed.
+__device__ __forceinline__ cds c_mul(cds a, float4 w) {
+  const float2 ah = un(a.h), al = un(a.l);
+  const float p1 = __fmul_rn(ah.x, w.x), p2 = __fmul_rn(-ah.y, w.y), p3 = __fmul_rn(ah.x, w.y), p4 = __fmul_rn(ah.y, w.x);
+  const float e1 = __fmaf_rn(ah.x, w.x, -p1), e2 = __fmaf_rn(-ah.y, w.y, -p2), e3 = __fmaf_rn(ah.x, w.y, -p3),
+              e4 = __fmaf_rn(ah.y, w.x, -p4);
+  const f2 p = pk(p1, p3), q = pk(p2, p4);
+  const f2 s = add2(p, q), v = sub2(s, p), t = add2(sub2(p, sub2(s, v)), sub2(q, v));
+  const float2 c = un(add2(t, add2(pk(e1, e3), pk(e2, e4))));
+  const float r = __fmaf_rn(-al.y, w.y, __fmaf_rn(-ah.y, w.w, __fmaf_rn(al.x, w.x, __fmaf_rn(ah.x, w.z, c.x))));
+  const float i = __fmaf_rn(al.y, w.x, __fmaf_rn(ah.y, w.z, __fmaf_rn(al.x, w.y, __fmaf_rn(ah.x, w.w, c.y))));
+  const f2 lo = pk(r, i), h = add2(s, lo);
+  return {h, sub2(lo, sub2(h, s))};
+}
+
+// a * c for a real double-single constant.
+__device__ __forceinline__ cds c_scale(cds a, float ch, float cl) {
+  const f2 c = pk(ch, ch), d = pk(cl, cl);
+  const f2 p = mul2(a.h, c), m = pk(-1.f, -1.f);
+  const f2 e = fma2(a.l, c, fma2(a.h, d, fma2(a.h, c, mul2(p, m))));
+  const f2 h = add2(p, e);
+  return {h, sub2(e, sub2(h, p))};
+}
+constexpr float kR2h = 0.707106769f, kR2l = 1.21016175e-08f;  // sqrt(1/2)
+__device__ __forceinline__ cds c_w8(cds a) { return c_scale(c_addi<1>(a, a), kR2h, kR2l); }     // a exp(2 pi i / 8)
+__device__ __forceinline__ cds c_w8c(cds a) { return c_scale(c_addi<-1>(a, a), -kR2h, -kR2l); }  // a exp(2 pi i 3 / 8)
+
+// Inverse DFTs of 2, 4, 8 and 16 points in registers, natural order in and out.
+// DFT4 of (x0, x1, x2, x3); I2: of (x0, x1, i x2, x3).
+template <bool I2 = false>
+__device__ __forceinline__ void dft4(cds &x0, cds &x1, cds &x2, cds &x3) {
+  const cds a = I2 ? c_addi<1>(x0, x2) : c_add(x0, x2), b = I2 ? c_addi<-1>(x0, x2) : c_sub(x0, x2);
+  const cds c = c_add(x1, x3), d = c_sub(x1, x3);
+  x0 = c_add(a, c);
+  x1 = c_addi<1>(b, d);
+  x2 = c_sub(a, c);
+  x3 = c_addi<-1>(b, d);
+}
+
+template <int R> struct Dft;
+template <> struct Dft<2> {
+  __device__ static __forceinline__ void run(cds *x) {
+    const cds a = c_add(x[0], x[1]);
+    x[1] = c_sub(x[0], x[1]);
+    x[0] = a;
+  }
+};
+template <> struct Dft<4> {
+  __device__ static __forceinline__ void run(cds *x) { dft4(x[0], x[1], x[2], x[3]); }
+};
+template <> struct Dft<8> {
+  __device__ static __forceinline__ void run(cds *x) {
+    cds s[4], d[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[j] = c_add(x[j], x[j + 4]);
+      d[j] = c_sub(x[j], x[j + 4]);
+    }
+    d[1] = c_w8(d[1]);
+    d[3] = c_w8c(d[3]);
+    dft4(s[0], s[1], s[2], s[3]);
+    dft4<true>(d[0], d[1], d[2], d[3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      x[2 * j] = s[j];
+      x[2 * j + 1] = d[j];
+    }
+  }
+};
+template <> struct Dft<16> {
+  __device__ static __forceinline__ void run(cds *x) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dft4(x[j], x[j + 4], x[j + 8], x[j + 12]);  // x[j + 4 k1]
+    // times exp(2 pi i j k1 / 16); j k1 = 4 is a factor i, taken by the next DFT4.  cos, sin of pi / 8:
+    constexpr float ch = 0.923879504f, cl = 2.83074897e-08f, sh = 0.382683426f, sl = 6.22335072e-09f;
+    x[5] = c_mul(x[5], make_float4(ch, sh, cl, sl));
+    x[9] = c_w8(x[9]);
+    x[13] = c_mul(x[13], make_float4(sh, ch, sl, cl));
+    x[6] = c_w8(x[6]);
+    x[14] = c_w8c(x[14]);
+    x[7] = c_mul(x[7], make_float4(sh, ch, sl, cl));
+    x[11] = c_w8c(x[11]);
+    x[15] = c_mul(x[15], make_float4(-ch, -sh, -cl, -sl));
+    dft4(x[0], x[1], x[2], x[3]);
+    dft4(x[4], x[5], x[6], x[7]);
+    dft4<true>(x[8], x[9], x[10], x[11]);
+    dft4(x[12], x[13], x[14], x[15]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)  // x[4 k1 + k2] holds X[k1 + 4 k2]: transpose
+#pragma unroll
+      for (int j = 0; j < k; ++j) {
+        const cds t = x[4 * k + j];
+        x[4 * k + j] = x[4 * j + k];
+        x[4 * j + k] = t;
+      }
+  }
+};
 
 // ---------------------------------------------------------------------------
-// Pass 1: row transforms.  Logical plane q of the input is the sum over
-// z < nsum of grid[q * qstride + z * plane]; rows of planes [q0, q0 + np) go to
-// buf[(q - q0) * plane + y * nx + x] with the chk sign applied on input.  One
-// CTA holds PTS points (PTS / nx rows).  For rows of 512 points or more the
-// slot of point n within its row has its low three bits XORed with a function
-// of bits 3-5 and of the top three bits of n: the small-span butterflies
-// (strides 2, 4 and 16 slots) and the bit-reversed reads of the epilogue then
-// touch eight different 16-byte bank groups per quarter warp.
+// Pass 1: row transforms of length L = 2^LX over CTAs of 4096 points (S = 4096 / L
+// rows, 256 threads).  L = R0 M0: radix R0 on points n = n1 M0 + m, times
+// exp(2 pi i m k1 / L); then radix 16 on what is left (M0 = 256: twice; M0 = 16:
+// once).  The point with digit k1 done and n left lies at k1 M0 + n, one slot of
+// padding every M0: the last pass's lanes run over k1.  Output k = k1 + R0 k2 +
+// 16 R0 k3.
+//
+// Logical plane q of the input is the sum over z < nsum of grid[q * qstride +
+// z * plane]; rows of planes [q0, q0 + np) go to buf[(q - q0) * plane + y * nx + x]
+// with the chk sign applied on input.
+//
+// SPLIT: rows of 8192 points as two 4096-point halves on two CTAs: the first
+// decimation-in-frequency stage, span 4096, is done while loading, half 0 taking
+// x[n] + x[n + 4096] (whose DFT is X[2k]) and half 1 taking (x[n] - x[n + 4096])
+// exp(2 pi i n / 8192) (DFT X[2k + 1]).  Half h's output k goes to slot
+// h 4096 + k of the row (whole lines; the last column pass takes the columns in
+// pairs from the halves).
 // ---------------------------------------------------------------------------
-constexpr int kColT = 512, kColPts = 4096, kColNPT = kColPts / kColT, kColSmem = (kColPts + 256) * 16,
-              kColSmem2 = (2 * kColPts + 128) * 16 + kColPts * 8;
+constexpr int kRowT = 256, kRowPts = 4096;
+template <int LX> struct RowGeom {
+  static constexpr int L = 1 << LX, R0 = LX >= 9 ? L / 256 : L / 16, M0 = L / R0, S = kRowPts / L,
+                       LP = L + R0, SMEM = S * LP * 16, LOG2M0 = LX >= 9 ? 8 : 4;
+};
 
-template <int PTS, int T>
-__global__ void __launch_bounds__(T, 1024 / T)
-k_dsfft_rows(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t q0, int np, int log2ny, int log2nx,
+template <int LX, bool SPLIT>
+__global__ void __launch_bounds__(kRowT, 2)
+k_dsfft_rows(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t q0, int np, int log2ny,
              float4 *__restrict__ buf) {
+  using G = RowGeom<LX>;
   extern __shared__ float4 sm[];
-  constexpr int LOG2PTS = PTS == 8192 ? 13 : 12;
-  const int ny = 1 << log2ny;
-  const int64_t plane = (int64_t)ny << log2nx;
-  const int log2S = LOG2PTS - log2nx;  // rows per CTA
-  const int64_t row0 = (int64_t)blockIdx.x << log2S;
-  const int64_t nrows = (int64_t)np << log2ny;
-  const bool swz = log2nx >= 9;
-  auto pos = [&](int n, int q) {
-    int m = n;
-    if (swz) {
-      const int j = (n >> 3) & 7;
-      m = n ^ ((j & 3) | ((j & 2) << 1)) ^ ((n >> (log2nx - 3)) & 7);
-    }
-    return (q << log2nx) + m;
-  };
-  if (nsum == 1) {
-    // all loads of the thread in flight before the first shared store
-    constexpr int K = PTS / T;
-    float2 gv[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int t = threadIdx.x + k * T;
-      const int q = t >> log2nx, x = t & ((1 << log2nx) - 1);
-      const int64_t R = row0 + q;
-      gv[k] = make_float2(0.f, 0.f);
-      if (R < nrows)
-        gv[k] = grid[(q0 + (R >> log2ny)) * qstride + ((int64_t)(R & (ny - 1)) << log2nx) + x];
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int t = threadIdx.x + k * T;
-      const int q = t >> log2nx, x = t & ((1 << log2nx) - 1);
-      const int y = (int)((row0 + q) & (ny - 1));
-      const float sg = ((x + y) & 1) ? -1.f : 1.f;
-      sm[pos(x, q)] = make_float4(sg * gv[k].x, 0.f, sg * gv[k].y, 0.f);
-    }
-  } else {
-  for (int t = threadIdx.x; t < PTS; t += T) {
-    const int q = t >> log2nx, x = t & ((1 << log2nx) - 1);
-    const int64_t R = row0 + q;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (R < nrows) {
-      const int64_t pl = R >> log2ny;
-      const int y = (int)(R & (ny - 1));
-      const float2 *src = grid + (q0 + pl) * qstride + ((int64_t)y << log2nx) + x;
-      float2 g = src[0];
-      dsf re = {g.x, 0.f}, im = {g.y, 0.f};
-      for (int z = 1; z < nsum; ++z) {
-        g = src[z * plane];
-        re = ds_add(re, {g.x, 0.f});
-        im = ds_add(im, {g.y, 0.f});
-      }
-      const float sg = ((x + y) & 1) ? -1.f : 1.f;
-      v = make_float4(sg * re.hi, sg * re.lo, sg * im.hi, sg * im.lo);
-    }
-    sm[pos(x, q)] = v;
-  }
-  }
-  // An all-zero tile (whole empty grid rows, common in w-stack slices)
-  // transforms to zero: write zeros and skip the arithmetic.
-  bool nz = false;
-  for (int t = threadIdx.x; t < PTS && !nz; t += T) {
-    const float4 v = sm[pos(t & ((1 << log2nx) - 1), t >> log2nx)];
-    nz = v.x != 0.f || v.z != 0.f;
-  }
-  if (!__syncthreads_or(nz)) {
-    for (int t = threadIdx.x; t < PTS; t += T) {
-      const int64_t R = row0 + (t >> log2nx);
-      if (R < nrows) buf[(R << log2nx) + (t & ((1 << log2nx) - 1))] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    return;
-  }
-  ds_dif_cta<T>(sm, log2nx, log2S, false, pos, TwGlobal());
-  for (int t = threadIdx.x; t < PTS; t += T) {
-    const int q = t >> log2nx, x = t & ((1 << log2nx) - 1);
-    const int64_t R = row0 + q;
-    if (R < nrows) buf[(R << log2nx) + x] = sm[pos(brev(x, log2nx), q)];
-  }
-}
-
-// 8192-point rows as two 4096-point halves on two CTAs (64 KiB of shared
-// memory each, so that two CTAs share an SM): the first decimation-in-
-// frequency stage, span 4096, is done while loading, CTA h = 0 taking
-// x[n] + x[n + 4096] (whose DFT is X[2k]) and h = 1 taking
-// (x[n] - x[n + 4096]) exp(2 pi i n / 8192) (DFT X[2k + 1]); each writes its
-// 4096 outputs to the even or odd positions of the row.
-__global__ void __launch_bounds__(512, 2)
-k_dsfft_rows_split(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t q0, int np, int log2ny,
-                   float4 *__restrict__ buf) {
-  extern __shared__ float4 sm[];
-  constexpr int LX = 13, LH = 12, H = 1 << LH;
-  const int ny = 1 << log2ny;
-  const int64_t plane = (int64_t)ny << LX;
-  const int64_t R = blockIdx.x >> 1;
-  const int half = blockIdx.x & 1;
-  auto pos = [&](int n, int) {
-    const int j = (n >> 3) & 7;
-    return n ^ ((j & 3) | ((j & 2) << 1)) ^ ((n >> (LH - 3)) & 7);
-  };
-  const int64_t pl = R >> log2ny;
-  const int y = (int)(R & (ny - 1));
-  const float2 *src = grid + (q0 + pl) * qstride + ((int64_t)y << LX);
-  auto in = [&](int x) -> float4 {
-    float2 g = src[x];
-    dsf re = {g.x, 0.f}, im = {g.y, 0.f};
+  constexpr int R0 = G::R0, M0 = G::M0, S = G::S, IT = 16 / R0, LROW = SPLIT ? LX + 1 : LX;
+  const int ny = 1 << log2ny, half = SPLIT ? blockIdx.x & 1 : 0;
+  const int64_t plane = (int64_t)ny << LROW, nrows = (int64_t)np << log2ny;
+  const int64_t row0 = SPLIT ? blockIdx.x >> 1 : (int64_t)blockIdx.x * S;
+  // one FP32 value of row q of this CTA, w-planes summed, signed
+  auto in = [&](int64_t R, int x) -> cds {
+    if (R >= nrows) return {0, 0};
+    const int y = (int)(R & (ny - 1));
+    const float2 *src = grid + (q0 + (R >> log2ny)) * qstride + ((int64_t)y << LROW) + x;
+    float2 g = src[0];
+    cds v{pk(g.x, g.y), 0};
     for (int z = 1; z < nsum; ++z) {
-      g = src[z * plane + x];
-      re = ds_add(re, {g.x, 0.f});
-      im = ds_add(im, {g.y, 0.f});
+      g = src[z * plane];
+      v = c_add(v, cds{pk(g.x, g.y), 0});
     }
     const float sg = ((x + y) & 1) ? -1.f : 1.f;
-    return make_float4(sg * re.hi, sg * re.lo, sg * im.hi, sg * im.lo);
+    return {mul2(v.h, pk(sg, sg)), mul2(v.l, pk(sg, sg))};
   };
-  if (nsum == 1) {
-    constexpr int K = H / 512;
-    float2 ga[K], gb[K];
+  cds x[16];
+  if (nsum == 1) {  // all loads in flight before any is used
+    float2 ga[16], gb[SPLIT ? 16 : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      ga[k] = src[threadIdx.x + k * 512];
-      gb[k] = src[threadIdx.x + k * 512 + H];
+    for (int j = 0; j < 16; ++j) {
+      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+      const int64_t R = row0 + q;
+      const float2 *src =
+          grid + (q0 + (R >> log2ny)) * qstride + ((R & (ny - 1)) << LROW) + (j % R0) * M0 + m;
+      ga[j] = R < nrows ? src[0] : make_float2(0.f, 0.f);
+      if (SPLIT) gb[SPLIT ? j : 0] = src[1 << LX];
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int n = threadIdx.x + k * 512;
-      const float sg = ((n + y) & 1) ? -1.f : 1.f;  // n and n + 4096 have the same parity
-      const float4 a = make_float4(sg * ga[k].x, 0.f, sg * ga[k].y, 0.f);
-      const float4 b = make_float4(sg * gb[k].x, 0.f, sg * gb[k].y, 0.f);
-      float4 v;
-      if (half == 0) {
-        v = c_add_nr(a, b);
-      } else {
-        v = c_add_nr(a, c_neg(b));
-        if (n) v = c_mul(v, twiddle(n, LX));
+    for (int j = 0; j < 16; ++j) {
+      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+      const float sg = ((m + (int)(row0 + q)) & 1) ? -1.f : 1.f;  // M0, ny and 4096 are even
+      x[j] = {mul2(pk(ga[j].x, ga[j].y), pk(sg, sg)), 0};
+      if (SPLIT) {
+        const float2 b = gb[SPLIT ? j : 0];
+        const cds y{mul2(pk(b.x, b.y), pk(sg, sg)), 0};
+        x[j] = half ? c_sub(x[j], y) : c_add(x[j], y);
       }
-      sm[pos(n, 0)] = v;
     }
   } else {
-  for (int n = threadIdx.x; n < H; n += 512) {
-    const float4 a = in(n), b = in(n + H);
-    float4 v;
-    if (half == 0) {
-      v = c_add_nr(a, b);
-    } else {
-      v = c_add_nr(a, c_neg(b));
-      if (n) v = c_mul(v, twiddle(n, LX));
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+      const int n = (j % R0) * M0 + m;
+      x[j] = in(row0 + q, n);
+      if (SPLIT) {
+        const cds y = in(row0 + q, n + (1 << LX));
+        x[j] = half ? c_sub(x[j], y) : c_add(x[j], y);
+      }
     }
-    sm[pos(n, 0)] = v;
   }
-  }
-  // An all-zero half (a whole empty grid row) transforms to zero.
+  // Rows (or the half's sums) that are all zero, common in w-stack slices, transform to zero.
   bool nz = false;
-  for (int n = threadIdx.x; n < H && !nz; n += 512) {
-    const float4 v = sm[pos(n, 0)];
-    nz = v.x != 0.f || v.z != 0.f;
-  }
-  float4 *out = buf + (R << LX) + half;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) nz = nz || (x[j].h & 0x7fffffff7fffffffull) != 0;
   if (!__syncthreads_or(nz)) {
-    for (int k = threadIdx.x; k < H; k += 512) out[2 * k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = threadIdx.x; t < kRowPts; t += kRowT) {
+      const int64_t R = row0 + (t >> LX);
+      if (R < nrows)
+        buf[(R << LROW) + (half << LX) + (t & (G::L - 1))] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     return;
   }
-  ds_dif_cta<512>(sm, LH, 0, false, pos, TwGlobal());
-  for (int k = threadIdx.x; k < H; k += 512) out[2 * k] = sm[pos(brev(k, LH), 0)];
+  if (SPLIT && half) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = c_mul(x[j], __ldg(&g_tw[(j * M0 + threadIdx.x) << (kLog2Tw - LROW)]));
+  }
+#pragma unroll
+  for (int j = 0; j < IT; ++j) {
+    const int item = threadIdx.x + j * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+    Dft<R0>::run(x + j * R0);
+    float4 *o = sm + q * G::LP + m;
+#pragma unroll
+    for (int k = 0; k < R0; ++k) {
+      const float4 *tw = M0 == 256 ? g_tw256 : g_tw16;
+      if (k) x[j * R0 + k] = c_mul(x[j * R0 + k], __ldg(&tw[k * (16 / R0) * M0 + m]));
+      o[k * (M0 + 1)] = c_to(x[j * R0 + k]);
+    }
+  }
+  __syncthreads();
+  if (M0 == 256) {  // radix 16 on n = n2 16 + m2, in place
+    const int m = threadIdx.x & 15, k1 = (threadIdx.x >> 4) % R0, q = (threadIdx.x >> 4) / R0;
+    float4 *o = sm + q * G::LP + k1 * (M0 + 1) + m;
+#pragma unroll
+    for (int n = 0; n < 16; ++n) x[n] = c_from(o[n * 16]);
+    Dft<16>::run(x);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) o[k * 16] = c_to(k ? c_mul(x[k], __ldg(&g_tw16[k * 16 + m])) : x[k]);
+    __syncthreads();
+  }
+  constexpr int KS = G::L / 16;  // outputs with the last digit 0
+  const int kk = threadIdx.x & (KS - 1), q = threadIdx.x / KS, k1 = kk % R0, k2 = kk / R0;
+  const float4 *o = sm + q * G::LP + k1 * (M0 + 1) + k2 * 16;
+#pragma unroll
+  for (int n = 0; n < 16; ++n) x[n] = c_from(o[n]);
+  Dft<16>::run(x);
+  const int64_t R = row0 + q;
+  if (R >= nrows) return;
+  float4 *out = buf + (R << LROW) + (half << LX) + kk;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) out[k * KS] = c_to(x[k]);
 }
 
 // ---------------------------------------------------------------------------
-// Column decomposition ny = N1 N2 (N1 <= N2 <= 128) and the CTA tiles.
+// Column DFTs of length N = 2^LN over CTA tiles of PTS = N S points (S sequences, T =
+// PTS / 16 threads): N <= 16 in registers; else radix R0 = N / 16 on n = n1 16 + m,
+// through shared memory at [k1 16 + m][q], then radix 16.  Lanes run over the
+// sequences (adjacent columns), so no access conflicts and the twiddles are one
+// per warp.  load(n, q) gives a point, out(i, k, q, v) takes output k (i = 0..15
+// numbers the thread's outputs); `sm` is free again after the last read's barrier,
+// which the caller places.
 // ---------------------------------------------------------------------------
+template <int LN, int LOG2PTS, typename Load, typename Out>
+__device__ __forceinline__ void col_dft(float4 *sm, Load load, Out out) {
+  constexpr int N = 1 << LN, LS = LOG2PTS - LN, S = 1 << LS, T = 1 << (LOG2PTS - 4);
+  cds x[16];
+  if constexpr (N <= 16) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = load(j % N, (int)threadIdx.x + (j / N) * T);
+#pragma unroll
+    for (int j = 0; j < 16 / N; ++j) {
+      Dft<N>::run(x + j * N);
+#pragma unroll
+      for (int k = 0; k < N; ++k) out(j * N + k, k, (int)threadIdx.x + j * T, x[j * N + k]);
+    }
+  } else {
+    constexpr int R0 = N / 16;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int item = threadIdx.x + (j / R0) * T;
+      x[j] = load((j % R0) * 16 + (item >> LS), item & (S - 1));
+    }
+#pragma unroll
+    for (int j = 0; j < 16 / R0; ++j) {
+      const int item = threadIdx.x + j * T, m = item >> LS, q = item & (S - 1);
+      Dft<R0>::run(x + j * R0);
+#pragma unroll
+      for (int k = 0; k < R0; ++k) {
+        if (k && m) x[j * R0 + k] = c_mul(x[j * R0 + k], __ldg(&g_tw16[k * (16 / R0) * 16 + m]));
+        sm[((k * 16 + m) << LS) + q] = c_to(x[j * R0 + k]);
+      }
+    }
+    __syncthreads();
+    const int q = threadIdx.x & (S - 1), k1 = threadIdx.x >> LS;
+#pragma unroll
+    for (int n = 0; n < 16; ++n) x[n] = c_from(sm[((k1 * 16 + n) << LS) + q]);
+    Dft<16>::run(x);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) out(k, k1 + R0 * k, q, x[k]);
+  }
+}
+
+// Column decomposition ny = N1 N2 (N1 <= N2 <= 128) and the CTA tiles.
 struct ColGeom {
   int log2N1, log2N2;
   int log2G1, log2WC1;  // cols1: n2 values x columns per CTA
-  int log2G2, log2WC2;  // cols2: k1 values x columns per CTA
+  int log2G2, log2WC2;  // cols2: k1 values x columns per CTA (half as many columns for w-stacking)
 };
 
 static bool col_geom(int log2ny, int log2nx, ColGeom *c) {
   c->log2N1 = log2ny / 2;
   c->log2N2 = log2ny - c->log2N1;
-  if (c->log2N2 > 7 || c->log2N1 < 2) return false;
+  if (c->log2N2 > 7 || c->log2N1 < 3) return false;
   const int lp = 12;  // log2 of the points per column CTA
   c->log2G1 = std::min(7 - c->log2N1, c->log2N2);
   c->log2WC1 = lp - c->log2N1 - c->log2G1;
@@ -408,42 +464,40 @@ static bool col_geom(int log2ny, int log2nx, ColGeom *c) {
   return c->log2WC1 <= log2nx && c->log2WC2 <= log2nx && c->log2WC1 >= 5 && c->log2WC2 >= 5;
 }
 
+constexpr int kColPts = 4096, kColT = 256, kWsPts = 2048, kWsT = 128;
+
+// Slot within a row of image column x: 8192-point rows come as two halves.
+__device__ __forceinline__ int col_slot(int x, int log2nx) {
+  return log2nx == 13 ? ((x & 1) << 12) + (x >> 1) : x;
+}
+
 // Pass 2: length-N1 DFTs over rows n2 + N2 n1, twiddled, in place.
-__global__ void __launch_bounds__(kColT)
+template <int LN>
+__global__ void __launch_bounds__(kColT, 2)
 k_dsfft_cols1(float4 *__restrict__ buf, int log2ny, int log2nx, ColGeom cg, int64_t ntile_pl) {
   extern __shared__ float4 sm[];
   const int64_t pl = blockIdx.x / ntile_pl;
   const int64_t t0 = blockIdx.x - pl * ntile_pl;
   const int ntx = 1 << (log2nx - cg.log2WC1);
   const int n2_0 = (int)(t0 / ntx) << cg.log2G1, x0 = (int)(t0 % ntx) << cg.log2WC1;
-  float4 *p = buf + (pl << (log2ny + log2nx));
-  const int WC1 = (1 << cg.log2WC1) - 1, log2S = cg.log2G1 + cg.log2WC1;
+  float4 *p = buf + (pl << (log2ny + log2nx)) + x0;
+  const int WC1 = (1 << cg.log2WC1) - 1;
   auto addr = [&](int n1, int q) {
     const int n2 = n2_0 + (q >> cg.log2WC1);
-    return ((int64_t)(n2 + (n1 << cg.log2N2)) << log2nx) + x0 + (q & WC1);
+    return ((int64_t)(n2 + (n1 << cg.log2N2)) << log2nx) + (q & WC1);
   };
-  auto pos = [&](int n, int q) { return (n << log2S) + q; };
-  float4 *stw = sm + kColPts;
-  stage_twiddles(stw, cg.log2N1);
-  // the 4-step twiddles exp(2 pi i n2 k1 / ny) of this CTA's G1 x N1 outputs
-  float4 *stw2 = stw + 128;
-  for (int e = threadIdx.x; e < (1 << (cg.log2G1 + cg.log2N1)); e += kColT)
-    stw2[e] = twiddle((n2_0 + (e >> cg.log2N1)) * (e & ((1 << cg.log2N1) - 1)), log2ny);
-  for (int t = threadIdx.x; t < kColPts; t += kColT) cp_async16(sm + t, p + addr(t >> log2S, t & ((1 << log2S) - 1)));
-  cp_async_wait_all();
-  __syncthreads();
-  ds_dif_cta<kColT>(sm, cg.log2N1, log2S, true, pos, TwShared{stw, cg.log2N1});
-  for (int t = threadIdx.x; t < kColPts; t += kColT) {
-    const int k1 = t >> log2S, q = t & ((1 << log2S) - 1);
-    const int g = q >> cg.log2WC1;
-    const float4 v = sm[pos(brev(k1, cg.log2N1), q)];
-    p[addr(k1, q)] = (n2_0 + g && k1) ? c_mul(v, stw2[(g << cg.log2N1) + k1]) : v;
-  }
+  col_dft<LN, 12>(
+      sm, [&](int n, int q) { return c_from(p[addr(n, q)]); },
+      [&](int, int k, int q, cds v) {
+        const int e = (n2_0 + (q >> cg.log2WC1)) * k;
+        p[addr(k, q)] = c_to(e ? c_mul(v, __ldg(&g_tw[e << (kLog2Tw - log2ny)])) : v);
+      });
 }
 
 // Pass 3 for invert_2d: length-N2 DFTs over rows N2 k1 + n2 -> row k1 + N1 k2;
 // image = part(v * chk * s0) * gcf [/ sumwt].  Plane pl is image b = b0 + pl.
-__global__ void __launch_bounds__(kColT)
+template <int LN>
+__global__ void __launch_bounds__(kColT, 2)
 k_dsfft_cols2_image(const float4 *__restrict__ buf, int log2ny, int log2nx, ColGeom cg, int64_t ntile_pl, int64_t b0,
                     float s0, const double *__restrict__ gcf, const double *__restrict__ sumwt,
                     double *__restrict__ im_re, double *__restrict__ im_im) {
@@ -453,20 +507,9 @@ k_dsfft_cols2_image(const float4 *__restrict__ buf, int log2ny, int log2nx, ColG
   const int ntx = 1 << (log2nx - cg.log2WC2);
   const int k1_0 = (int)(t0 / ntx) << cg.log2G2, x0 = (int)(t0 % ntx) << cg.log2WC2;
   const float4 *p = buf + (pl << (log2ny + log2nx));
-  const int WC2 = (1 << cg.log2WC2) - 1, log2S = cg.log2G2 + cg.log2WC2, S1 = (1 << log2S) - 1;
+  const int WC2 = (1 << cg.log2WC2) - 1;
   const int64_t b = b0 + pl;
   const int64_t obase = b << (log2ny + log2nx);
-  auto pos = [&](int n, int q) { return (n << log2S) + q; };
-  for (int t = threadIdx.x; t < kColPts; t += kColT) {
-    const int n2 = t >> log2S, q = t & S1;
-    const int k1 = k1_0 + (q >> cg.log2WC2);
-    cp_async16(sm + t, p + ((int64_t)((k1 << cg.log2N2) + n2) << log2nx) + x0 + (q & WC2));
-  }
-  cp_async_wait_all();
-  float4 *stw = sm + kColPts;
-  stage_twiddles(stw, cg.log2N2);
-  __syncthreads();
-  ds_dif_cta<kColT>(sm, cg.log2N2, log2S, true, pos, TwShared{stw, cg.log2N2});
   double inv = 1.0;
   bool zero = false;
   if (sumwt) {
@@ -474,102 +517,114 @@ k_dsfft_cols2_image(const float4 *__restrict__ buf, int log2ny, int log2nx, ColG
     zero = !(w > 0.0);
     inv = zero ? 0.0 : 1.0 / w;
   }
-  for (int t = threadIdx.x; t < kColPts; t += kColT) {
-    const int k2 = t >> log2S, q = t & S1;
-    const float4 v = sm[pos(brev(k2, cg.log2N2), q)];
-    const int k = k1_0 + (q >> cg.log2WC2) + (k2 << cg.log2N1), x = x0 + (q & WC2);
-    const int64_t o = obase + ((int64_t)k << log2nx) + x;
-    const double f = (double)((((x + k) & 1) ? -1.f : 1.f) * s0) * gcf[o];
-    double re = ds_to_double({v.x, v.y}) * f, im = ds_to_double({v.z, v.w}) * f;
-    if (sumwt) {
-      re = zero ? 0.0 : re * inv;
-      im = zero ? 0.0 : im * inv;
-    }
-    im_re[o] = re;
-    if (im_im) im_im[o] = im;
-  }
+  col_dft<LN, 12>(
+      sm,
+      [&](int n, int q) {
+        const int k1 = k1_0 + (q >> cg.log2WC2);
+        return c_from(p[((int64_t)((k1 << cg.log2N2) + n) << log2nx) + col_slot(x0 + (q & WC2), log2nx)]);
+      },
+      [&](int, int k2, int q, cds c) {
+        const float4 v = c_to(c);
+        const int k = k1_0 + (q >> cg.log2WC2) + (k2 << cg.log2N1), x = x0 + (q & WC2);
+        const int64_t o = obase + ((int64_t)k << log2nx) + x;
+        const double f = (double)((((x + k) & 1) ? -1.f : 1.f) * s0) * gcf[o];
+        double re = ds_to_double({v.x, v.z}) * f, im = ds_to_double({v.y, v.w}) * f;
+        if (sumwt) {
+          re = zero ? 0.0 : re * inv;
+          im = zero ? 0.0 : im * inv;
+        }
+        im_re[o] = re;
+        if (im_im) im_im[o] = im;
+      });
+}
+
+// Re(exp(-2 pi i w nterm) v) as a double-single number; nt.hi < 0 marks pixels beyond the horizon (0).
+__device__ __forceinline__ dsf wscreen_re(float2 nt, dsf w, cds c) {
+  const dsf t = ds_mul(w, {nt.x, nt.y});
+  // turns reduced to [-1/2, 1/2], then the quadrant: roundings through the 1.5 2^23 shift
+  const float big = 12582912.f;
+  const float r = fabsf(t.hi) < 4.0e6f ? __fsub_rn(__fadd_rn(t.hi, big), big) : rintf(t.hi);
+  const float f = __fadd_rn(__fsub_rn(t.hi, r), t.lo);
+  const float q4 = __fmaf_rn(f, 4.f, big);
+  float cs, sn;
+  sincos_quadrant(__fmaf_rn(__fsub_rn(q4, big), -2.f, 8.f * f), __float_as_uint(q4) & 3u, &cs, &sn);
+  // cos re + sin im
+  const float4 v = c_to(c);
+  const dsf p = two_prod(v.x, cs), q = two_prod(v.y, sn), s = two_sum(p.hi, q.hi);
+  const float e = __fmaf_rn(v.w, sn, __fmaf_rn(v.z, cs, __fadd_rn(s.lo, __fadd_rn(p.lo, q.lo))));
+  return nt.x < 0.f ? dsf{0.f, 0.f} : dsf{s.hi, e};
 }
 
 // Pass 3 for w-stacking: planes [p0, p1) of the flattened (image b, slice s)
 // order, buf holding them from p0.  Each CTA sums Re(wb_s v) over the slices
 // of its tile into double-single accumulators and adds them to the image's DS
 // slots (image memory viewed as float2; the group holding slice 0 of image b
-// writes them).
-__global__ void __launch_bounds__(kColT)
+// writes them).  Tiles of 2048 points on 128 threads: 16 accumulators a
+// thread, and three CTAs share an SM, one's loads under the others' arithmetic; the
+// sums and the w-screen terms wait in shared memory, each in its thread's own slots
+// (in registers the sums spilled).
+template <int LN>
+__global__ void __launch_bounds__(kWsT, 3)
 k_dsfft_cols2_wstack(const float4 *__restrict__ buf, int log2ny, int log2nx, ColGeom cg, int64_t p0, int64_t p1,
                      int K, double fov, const double *__restrict__ wmean, float2 *__restrict__ slots) {
   extern __shared__ float4 sm[];
-  const int ntx = 1 << (log2nx - cg.log2WC2);
-  const int k1_0 = (int)(blockIdx.x / ntx) << cg.log2G2, x0 = (int)(blockIdx.x % ntx) << cg.log2WC2;
-  const int WC2 = (1 << cg.log2WC2) - 1, log2S = cg.log2G2 + cg.log2WC2, S1 = (1 << log2S) - 1;
-  const int n = 1 << log2nx;
+  constexpr int TILE = (1 << LN) > 16 ? kWsPts : 0;
+  float2 *snt = reinterpret_cast<float2 *>(sm + TILE);  // per-pixel w-screen terms, [i][thread]
+  const int lwc = cg.log2WC2 - 1, ntx = 1 << (log2nx - lwc);
+  const int k1_0 = (int)(blockIdx.x / ntx) << cg.log2G2, x0 = (int)(blockIdx.x % ntx) << lwc;
+  const int WC = (1 << lwc) - 1, n = 1 << log2nx;
   const dsf c2 = ds_from_double(fov * fov / ((double)n * n));
-  auto pos = [&](int k, int q) { return (k << log2S) + q; };
-  // Two tiles: the next slice's tile is copied in while this one is
-  // transformed.
-  float4 *stw = sm + 2 * kColPts;
-  stage_twiddles(stw, cg.log2N2);  // ordered before first use by the barrier after the first load
-  float2 *snt = reinterpret_cast<float2 *>(stw + 128);  // kColPts per-pixel w-screen terms
-  auto issue = [&](int64_t pp, float4 *dst) {
-    const float4 *p = buf + ((pp - p0) << (log2ny + log2nx));
-    for (int t = threadIdx.x; t < kColPts; t += kColT) {
-      const int n2 = t >> log2S, q = t & S1;
-      const int k1 = k1_0 + (q >> cg.log2WC2);
-      cp_async16(dst + t, p + ((int64_t)((k1 << cg.log2N2) + n2) << log2nx) + x0 + (q & WC2));
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  float2 *sacc = snt + kWsPts;  // and the sums
+  // the image pixel of the thread's output i
+  auto pixel = [&](int i, int *k, int *x) {
+    constexpr int N = 1 << LN, LS = 11 - LN, S = 1 << LS;
+    const int q = N <= 16 ? (int)threadIdx.x + (i / N) * kWsT : threadIdx.x & (S - 1);
+    const int k2 = N <= 16 ? i % N : (int)(threadIdx.x >> LS) + (N / 16) * i;
+    *k = k1_0 + (q >> lwc) + (k2 << cg.log2N1);
+    *x = x0 + (q & WC);
   };
-  dsf acc[kColNPT];
-#pragma unroll
-  for (int m = 0; m < kColNPT; ++m) acc[m] = {0.f, 0.f};
-  issue(p0, sm);
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i) {
+    int k, x;
+    pixel(i, &k, &x);
+    const DsPix px = ds_wpix(k, x, n, c2);
+    // nterm, or hi = -1 where r^2 >= 1
+    snt[i * kWsT + threadIdx.x] = px.state == 2 ? make_float2(-1.f, 0.f) : make_float2(px.nterm.hi, px.nterm.lo);
+    sacc[i * kWsT + threadIdx.x] = make_float2(0.f, 0.f);
+  }
   for (int64_t pp = p0; pp < p1; ++pp) {
     const int64_t b = pp / K;
-    const int s = (int)(pp - b * K);
-    float4 *cur = ((pp - p0) & 1) ? sm + kColPts : sm;
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();  // this tile has landed, and every thread is done with the other one
-    if (pp + 1 < p1) issue(pp + 1, ((pp - p0) & 1) ? sm : sm + kColPts);
-    ds_dif_cta<kColT>(cur, cg.log2N2, log2S, true, pos, TwShared{stw, cg.log2N2});
-    const dsf w = ds_from_double(wmean[s]);
-#pragma unroll
-    for (int m = 0; m < kColNPT; ++m) {
-      const int t = threadIdx.x + m * kColT;
-      const int k2 = t >> log2S, q = t & S1;
-      const float4 v = cur[pos(brev(k2, cg.log2N2), q)];
-      // w-screen term of this thread's pixel t, formed at the first slice and
-      // kept in the thread's own shared slot: nterm, or hi = -1 where r^2 >= 1
-      if (pp == p0) {
-        const int k = k1_0 + (q >> cg.log2WC2) + (k2 << cg.log2N1), x = x0 + (q & WC2);
-        const DsPix px = ds_wpix(k, x, n, c2);
-        snt[t] = px.state == 2 ? make_float2(-1.f, 0.f) : make_float2(px.nterm.hi, px.nterm.lo);
-      }
-      const float2 nt = snt[t];
-      DsPix px;
-      px.state = nt.x < 0.f ? 2 : 1;
-      px.nterm = {nt.x, nt.y};
-      const float2 wb = ds_wbeam(px, w);
-      // Re(wb v) = wb.re v.re - wb.im v.im
-      acc[m] = ds_add(acc[m], ds_sub(ds_mul_f({v.x, v.y}, wb.x), ds_mul_f({v.z, v.w}, wb.y)));
-    }
+    const dsf w = ds_from_double(wmean[pp - b * K]);
+    const float4 *p = buf + ((pp - p0) << (log2ny + log2nx));
+    col_dft<LN, 11>(
+        sm,
+        [&](int n2, int q) {
+          const int k1 = k1_0 + (q >> lwc);
+          return c_from(p[((int64_t)((k1 << cg.log2N2) + n2) << log2nx) + col_slot(x0 + (q & WC), log2nx)]);
+        },
+        [&](int i, int, int, cds v) {
+          float2 &sum = sacc[i * kWsT + threadIdx.x];
+          const dsf a = ds_add({sum.x, sum.y}, wscreen_re(snt[i * kWsT + threadIdx.x], w, v));
+          sum = make_float2(a.hi, a.lo);
+        });
     if (pp + 1 == p1 || (pp + 1) / K != b) {
       const bool first = p0 <= b * K;
-      float2 *out = slots + (b << (log2ny + log2nx));
-#pragma unroll
-      for (int m = 0; m < kColNPT; ++m) {
-        const int t = threadIdx.x + m * kColT;
-        const int k2 = t >> log2S, q = t & S1;
-        const int k = k1_0 + (q >> cg.log2WC2) + (k2 << cg.log2N1), x = x0 + (q & WC2);
-        float2 *o = out + ((int64_t)k << log2nx) + x;
-        dsf v = acc[m];
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        int k, x;
+        pixel(i, &k, &x);
+        float2 *o = slots + (b << (log2ny + log2nx)) + ((int64_t)k << log2nx) + x;
+        float2 &sum = sacc[i * kWsT + threadIdx.x];
+        dsf a{sum.x, sum.y};
         if (!first) {
           const float2 old = *o;
-          v = ds_add(v, {old.x, old.y});
+          a = ds_add(a, {old.x, old.y});
         }
-        *o = make_float2(v.hi, v.lo);
-        acc[m] = {0.f, 0.f};
+        *o = make_float2(a.hi, a.lo);
+        sum = make_float2(0.f, 0.f);
       }
     }
+    __syncthreads();  // the exchange area is free for the next plane
   }
 }
 
@@ -606,6 +661,23 @@ bool dsfft_supported(int ny, int nx) {
   return col_geom(ly, lx, &cg);
 }
 
+// Shared memory of the column kernels: the exchange tile where N > 16; the w-screen terms and sums.
+static size_t col_smem(int log2N, bool wstack) {
+  if (wstack) return (log2N > 4 ? kWsPts * 16 : 0) + kWsPts * 16;
+  return log2N > 4 ? kColPts * 16 : 0;
+}
+
+// Calls f(std::integral_constant<int, V>) for the V of [LO, HI] that equals v.
+template <int LO, int HI, typename F>
+static void with_const(int v, F f) {
+  if constexpr (LO <= HI) {
+    if (v == LO)
+      f(std::integral_constant<int, LO>());
+    else
+      with_const<LO + 1, HI>(v, f);
+  }
+}
+
 // Function attributes belong to each device's context: set once per device.
 static int set_smem() {
   static std::atomic<unsigned> done{0};
@@ -613,11 +685,21 @@ static int set_smem() {
   ARL_CUDA(cudaGetDevice(&dev));
   const unsigned bit = 1u << (dev & 31);
   if (done.load() & bit) return ARLGPU_OK;
-  ARL_CUDA(cudaFuncSetAttribute(k_dsfft_rows_split, cudaFuncAttributeMaxDynamicSharedMemorySize, 4096 * 16));
-  ARL_CUDA(cudaFuncSetAttribute(k_dsfft_rows<4096, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4096 * 16));
-  ARL_CUDA(cudaFuncSetAttribute(k_dsfft_cols1, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
-  ARL_CUDA(cudaFuncSetAttribute(k_dsfft_cols2_image, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
-  ARL_CUDA(cudaFuncSetAttribute(k_dsfft_cols2_wstack, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem2));
+  cudaError_t e = cudaSuccess;
+  auto set = [&](const void *f, size_t bytes) {
+    const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (r != cudaSuccess) e = r;
+  };
+  for (int l = 6; l <= 12; ++l)
+    with_const<6, 12>(l, [&](auto c) { set((const void *)k_dsfft_rows<c.value, false>, RowGeom<c.value>::SMEM); });
+  set((const void *)k_dsfft_rows<12, true>, RowGeom<12>::SMEM);
+  for (int l = 3; l <= 7; ++l)
+    with_const<3, 7>(l, [&](auto c) {
+      set((const void *)k_dsfft_cols1<c.value>, col_smem(l, false));
+      set((const void *)k_dsfft_cols2_image<c.value>, col_smem(l, false));
+      set((const void *)k_dsfft_cols2_wstack<c.value>, col_smem(l, true));
+    });
+  ARL_CUDA(e);
   done.fetch_or(bit);
   return ARLGPU_OK;
 }
@@ -627,15 +709,21 @@ static int rows_cols1(const float2 *grid, int64_t qstride, int nsum, int64_t q0,
                       const ColGeom &cg, float4 *buf, cudaStream_t st) {
   const int64_t nrows = np << ly;
   if (lx == 13) {
-    k_dsfft_rows_split<<<(unsigned)(2 * nrows), 512, 4096 * 16, st>>>(grid, qstride, nsum, q0, (int)np, ly, buf);
+    k_dsfft_rows<12, true><<<(unsigned)(2 * nrows), kRowT, RowGeom<12>::SMEM, st>>>(grid, qstride, nsum, q0, (int)np,
+                                                                                   ly, buf);
   } else {
     const int log2S = 12 - lx;
     const int64_t rblocks = (nrows + ((int64_t)1 << log2S) - 1) >> log2S;
-    k_dsfft_rows<4096, 512><<<(unsigned)rblocks, 512, 4096 * 16, st>>>(grid, qstride, nsum, q0, (int)np, ly, lx, buf);
+    with_const<6, 12>(lx, [&](auto c) {
+      k_dsfft_rows<c.value, false><<<(unsigned)rblocks, kRowT, RowGeom<c.value>::SMEM, st>>>(grid, qstride, nsum, q0,
+                                                                                            (int)np, ly, buf);
+    });
   }
   ARL_LAUNCH_CHECK();
   const int64_t ntile = ((int64_t)1 << (cg.log2N2 - cg.log2G1)) << (lx - cg.log2WC1);
-  k_dsfft_cols1<<<(unsigned)(np * ntile), kColT, kColSmem, st>>>(buf, ly, lx, cg, ntile);
+  with_const<3, 7>(cg.log2N1, [&](auto c) {
+    k_dsfft_cols1<c.value><<<(unsigned)(np * ntile), kColT, col_smem(cg.log2N1, false), st>>>(buf, ly, lx, cg, ntile);
+  });
   ARL_LAUNCH_CHECK();
   count_launch(2);
   return ARLGPU_OK;
@@ -655,8 +743,10 @@ int dsfft_g2i_2d(const float2 *grid, int nb, int nw, int ny, int nx, const doubl
   ARL_TRY(rows_cols1(grid, plane * nw, nw, 0, nb, ly, lx, cg, b4, st));
   const int64_t ntile = ((int64_t)1 << (cg.log2N1 - cg.log2G2)) << (lx - cg.log2WC2);
   const float s0 = (((nx / 2) + (ny / 2)) & 1) ? -1.f : 1.f;
-  k_dsfft_cols2_image<<<(unsigned)(nb * ntile), kColT, kColSmem, st>>>(b4, ly, lx, cg, ntile, 0, s0, gcf, sumwt,
-                                                                          im_re, im_im);
+  with_const<3, 7>(cg.log2N2, [&](auto c) {
+    k_dsfft_cols2_image<c.value><<<(unsigned)(nb * ntile), kColT, col_smem(cg.log2N2, false), st>>>(
+        b4, ly, lx, cg, ntile, 0, s0, gcf, sumwt, im_re, im_im);
+  });
   ARL_LAUNCH_CHECK();
   count_launch(1);
   return ARLGPU_OK;
@@ -675,12 +765,14 @@ int dsfft_g2i_wstack(const float2 *grid, int nb, int K, int ny, int nx, double f
   ARL_TRY(set_smem());
   const int64_t plane = (int64_t)ny * nx, nplanes = (int64_t)nb * K;
   float4 *b4 = static_cast<float4 *>(buf);
-  const int64_t ntile = ((int64_t)1 << (cg.log2N1 - cg.log2G2)) << (lx - cg.log2WC2);
+  const int64_t ntile = ((int64_t)1 << (cg.log2N1 - cg.log2G2)) << (lx - cg.log2WC2 + 1);
   for (int64_t p0 = 0; p0 < nplanes; p0 += G) {
     const int64_t np = std::min(G, nplanes - p0);
     ARL_TRY(rows_cols1(grid, plane, 1, p0, np, ly, lx, cg, b4, st));
-    k_dsfft_cols2_wstack<<<(unsigned)ntile, kColT, kColSmem2, st>>>(b4, ly, lx, cg, p0, p0 + np, K, fov, wmean,
-                                                                      reinterpret_cast<float2 *>(image));
+    with_const<3, 7>(cg.log2N2, [&](auto c) {
+      k_dsfft_cols2_wstack<c.value><<<(unsigned)ntile, kWsT, col_smem(cg.log2N2, true), st>>>(
+          b4, ly, lx, cg, p0, p0 + np, K, fov, wmean, reinterpret_cast<float2 *>(image));
+    });
     ARL_LAUNCH_CHECK();
     count_launch(1);
   }

@@ -88,6 +88,25 @@ __device__ __forceinline__ dsf ds_from_double(double x) {
 
 __device__ __forceinline__ double ds_to_double(dsf a) { return (double)a.hi + (double)a.lo; }
 
+// cos and sin of (q + y / 2) quarter turns, |y| <= 1: y is the offset from
+// quadrant q's centre in eighths of a turn.  Least-maximum fits of sin(pi y / 4) / y
+// (degree 3 in y^2, 2.4e-9) and cos(pi y / 4) (degree 4, 5e-11), made for these
+// intervals; pi / 4 is split so that its rounding does not scale the sine.
+__device__ __forceinline__ void sincos_quadrant(float y, unsigned q, float *c, float *s) {
+  const float z = y * y;
+  float a = fmaf(z, -3.59545078e-05f, 2.49000713e-03f);
+  a = fmaf(a, z, -8.07454348e-02f);
+  a = fmaf(a, z, -2.4e-08f);  // pi / 4 = 0.78539818525 - 2.19e-8, less the fit's -2.1e-9
+  const float sn = fmaf(y, 0.78539818525f, y * a);
+  float b = fmaf(z, 3.52981134e-06f, -3.25938614e-04f);
+  b = fmaf(b, z, 1.58543252e-02f);
+  b = fmaf(b, z, -3.08425135e-01f);
+  const float cs = fmaf(b, z, 1.f);
+  const float cc = (q & 1) ? sn : cs, ss = (q & 1) ? cs : sn;
+  *c = __int_as_float(__float_as_int(cc) ^ (((q + 1) & 2) << 30));
+  *s = __int_as_float(__float_as_int(ss) ^ ((q & 2) << 30));
+}
+
 // w-screen phase of create_w_term_like at one pixel, in double-single:
 // nterm = 1 - sqrt(1 - r^2), r^2 = c2 ((y - n/2)^2 + (x - n/2)^2) with
 // c2 = fov^2 / n^2 (split from FP64).  The subtraction loses relative accuracy
