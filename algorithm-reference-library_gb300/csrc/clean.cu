@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "dsmath.cuh"
 
 namespace arlgpu {
 
@@ -68,19 +69,6 @@ constexpr unsigned long long kAbsMask = 0x7fffffffffffffffull;
 constexpr int kHogCopies = 16;
 constexpr int kHogPoll = 5;         // slots a polling lane reads: up to 160 CTAs
 constexpr int kHogTries = 1 << 20;  // rounds of polling (about a microsecond each) before a CTA gives up
-
-// a / b for y = 1 / b rounded to nearest: after a correction step the quotient is
-// within an ulp, and after a second one it is the rounded quotient (Markstein, IBM
-// J. Res. Dev. 34, 1990, pp. 111-119).  Five dependent operations; the peak's
-// component is on every CTA's path.  Outside the range where no step under- or
-// overflows, the division itself.
-__device__ __forceinline__ double hog_quotient(double a, double b, double y) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
-  if (ea < 1023 - 800 || ea > 1023 + 800 || eb < 1023 - 100 || eb > 1023 + 100) return __ddiv_rn(a, b);
-  double q = __dmul_rn(a, y);
-  q = fma(fma(-b, q, a), y, q);
-  return fma(fma(-b, q, a), y, q);
-}
 
 __device__ __forceinline__ void hog_put(unsigned long long *p, unsigned long long a, unsigned long long b) {
   asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
@@ -335,7 +323,7 @@ k_hogbom(HogArgs a) {
         __threadfence();
         r = *(volatile double *)&a.lookup[(size_t)buf * G + seg % G];
       }
-      s_mval = hog_quotient(__dmul_rn(r, a.gain), a.pmax, rcp);
+      s_mval = rounded_quotient(__dmul_rn(r, a.gain), a.pmax, rcp);
     }
     // The patch (overlapIndices of the reference): rows [r0, r1), columns [c0, c1), PSF pixel (x - mx + wx, y - my + wy).
     const long long r0 = max(0ll, mx - wx), r1 = min(a.nx, mx + wx);

@@ -35,7 +35,7 @@
 //     the same lane rate as single ones, for half the issue slots.
 // Radix-4 passes of run-time length, one butterfly a thread through shared
 // memory, were at 3.15 ms a plane of 8192^2 (w-stack, 32 planes: rows 1.20, cols1
-// 0.74, cols2 1.20 ms); now 1.92 ms (0.62, 0.56, 0.73).
+// 0.74, cols2 1.20 ms); now 1.80 ms (0.62, 0.54, 0.63).
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -405,7 +405,9 @@ k_dsfft_rows(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t
 // numbers the thread's outputs); `sm` is free again after the last read's barrier,
 // which the caller places.
 // ---------------------------------------------------------------------------
-template <int LN, int LOG2PTS, typename Load, typename Out>
+// HALVES: the exchange goes in two steps, high parts, then low parts, through half the
+// shared memory.
+template <int LN, int LOG2PTS, bool HALVES = false, typename Load, typename Out>
 __device__ __forceinline__ void col_dft(float4 *sm, Load load, Out out) {
   constexpr int N = 1 << LN, LS = LOG2PTS - LN, S = 1 << LS, T = 1 << (LOG2PTS - 4);
   cds x[16];
@@ -432,13 +434,32 @@ __device__ __forceinline__ void col_dft(float4 *sm, Load load, Out out) {
 #pragma unroll
       for (int k = 0; k < R0; ++k) {
         if (k && m) x[j * R0 + k] = c_mul(x[j * R0 + k], __ldg(&g_tw16[k * (16 / R0) * 16 + m]));
-        sm[((k * 16 + m) << LS) + q] = c_to(x[j * R0 + k]);
+        if (HALVES)
+          reinterpret_cast<f2 *>(sm)[((k * 16 + m) << LS) + q] = x[j * R0 + k].h;
+        else
+          sm[((k * 16 + m) << LS) + q] = c_to(x[j * R0 + k]);
       }
     }
     __syncthreads();
     const int q = threadIdx.x & (S - 1), k1 = threadIdx.x >> LS;
+    if (HALVES) {
+      f2 *sh = reinterpret_cast<f2 *>(sm);
+      f2 h[16];
 #pragma unroll
-    for (int n = 0; n < 16; ++n) x[n] = c_from(sm[((k1 * 16 + n) << LS) + q]);
+      for (int n = 0; n < 16; ++n) h[n] = sh[((k1 * 16 + n) << LS) + q];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int item = threadIdx.x + (j / R0) * T;
+        sh[(((j % R0) * 16 + (item >> LS)) << LS) + (item & (S - 1))] = x[j].l;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int n = 0; n < 16; ++n) x[n] = {h[n], sh[((k1 * 16 + n) << LS) + q]};
+    } else {
+#pragma unroll
+      for (int n = 0; n < 16; ++n) x[n] = c_from(sm[((k1 * 16 + n) << LS) + q]);
+    }
     Dft<16>::run(x);
 #pragma unroll
     for (int k = 0; k < 16; ++k) out(k, k1 + R0 * k, q, x[k]);
@@ -448,8 +469,8 @@ __device__ __forceinline__ void col_dft(float4 *sm, Load load, Out out) {
 // Column decomposition ny = N1 N2 (N1 <= N2 <= 128) and the CTA tiles.
 struct ColGeom {
   int log2N1, log2N2;
-  int log2G1, log2WC1;  // cols1: n2 values x columns per CTA
-  int log2G2, log2WC2;  // cols2: k1 values x columns per CTA (half as many columns for w-stacking)
+  int log2G1, log2WC1;  // cols1: n2 values x columns per 4096 points (the 2048-point tiles: half the columns)
+  int log2G2, log2WC2;  // cols2: k1 values x columns, likewise
 };
 
 static bool col_geom(int log2ny, int log2nx, ColGeom *c) {
@@ -471,25 +492,30 @@ __device__ __forceinline__ int col_slot(int x, int log2nx) {
   return log2nx == 13 ? ((x & 1) << 12) + (x >> 1) : x;
 }
 
-// Pass 2: length-N1 DFTs over rows n2 + N2 n1, twiddled, in place.
+// Pass 2: length-N1 DFTs over rows n2 + N2 n1, twiddled, in place.  Tiles of 2048
+// points on 128 threads, four CTAs an SM (this pass moves 32 bytes a point for some
+// 180 operations, near the machine's balance; it waits on its loads a third of the
+// time).  32 planes of 8192^2: 17.4 ms; the same with five CTAs, 18.0 with two of
+// 256 threads, 22.5 with resident CTAs that copy their next tile into shared memory
+// under the arithmetic.
 template <int LN>
-__global__ void __launch_bounds__(kColT, 2)
+__global__ void __launch_bounds__(kWsT, 4)
 k_dsfft_cols1(float4 *__restrict__ buf, int log2ny, int log2nx, ColGeom cg, int64_t ntile_pl) {
   extern __shared__ float4 sm[];
   const int64_t pl = blockIdx.x / ntile_pl;
   const int64_t t0 = blockIdx.x - pl * ntile_pl;
-  const int ntx = 1 << (log2nx - cg.log2WC1);
-  const int n2_0 = (int)(t0 / ntx) << cg.log2G1, x0 = (int)(t0 % ntx) << cg.log2WC1;
+  const int lwc = cg.log2WC1 - 1, ntx = 1 << (log2nx - lwc);
+  const int n2_0 = (int)(t0 / ntx) << cg.log2G1, x0 = (int)(t0 % ntx) << lwc;
   float4 *p = buf + (pl << (log2ny + log2nx)) + x0;
-  const int WC1 = (1 << cg.log2WC1) - 1;
+  const int WC1 = (1 << lwc) - 1;
   auto addr = [&](int n1, int q) {
-    const int n2 = n2_0 + (q >> cg.log2WC1);
+    const int n2 = n2_0 + (q >> lwc);
     return ((int64_t)(n2 + (n1 << cg.log2N2)) << log2nx) + (q & WC1);
   };
-  col_dft<LN, 12>(
+  col_dft<LN, 11>(
       sm, [&](int n, int q) { return c_from(p[addr(n, q)]); },
       [&](int, int k, int q, cds v) {
-        const int e = (n2_0 + (q >> cg.log2WC1)) * k;
+        const int e = (n2_0 + (q >> lwc)) * k;
         p[addr(k, q)] = c_to(e ? c_mul(v, __ldg(&g_tw[e << (kLog2Tw - log2ny)])) : v);
       });
 }
@@ -559,16 +585,17 @@ __device__ __forceinline__ dsf wscreen_re(float2 nt, dsf w, cds c) {
 // order, buf holding them from p0.  Each CTA sums Re(wb_s v) over the slices
 // of its tile into double-single accumulators and adds them to the image's DS
 // slots (image memory viewed as float2; the group holding slice 0 of image b
-// writes them).  Tiles of 2048 points on 128 threads: 16 accumulators a
-// thread, and three CTAs share an SM, one's loads under the others' arithmetic; the
-// sums and the w-screen terms wait in shared memory, each in its thread's own slots
-// (in registers the sums spilled).
+// writes them).  Tiles of 2048 points on 128 threads, and four CTAs share an SM,
+// one's loads under the others' arithmetic; the sums and the w-screen terms wait in
+// shared memory, each in its thread's own slots (in registers the sums spilled), and
+// the exchange takes half a tile at a time to leave them the room: 20.1 ms for 32
+// planes of 8192^2 against 23.3 ms with a whole tile and three CTAs.
 template <int LN>
-__global__ void __launch_bounds__(kWsT, 3)
+__global__ void __launch_bounds__(kWsT, 4)
 k_dsfft_cols2_wstack(const float4 *__restrict__ buf, int log2ny, int log2nx, ColGeom cg, int64_t p0, int64_t p1,
                      int K, double fov, const double *__restrict__ wmean, float2 *__restrict__ slots) {
   extern __shared__ float4 sm[];
-  constexpr int TILE = (1 << LN) > 16 ? kWsPts : 0;
+  constexpr int TILE = (1 << LN) > 16 ? kWsPts / 2 : 0;
   float2 *snt = reinterpret_cast<float2 *>(sm + TILE);  // per-pixel w-screen terms, [i][thread]
   const int lwc = cg.log2WC2 - 1, ntx = 1 << (log2nx - lwc);
   const int k1_0 = (int)(blockIdx.x / ntx) << cg.log2G2, x0 = (int)(blockIdx.x % ntx) << lwc;
@@ -596,7 +623,7 @@ k_dsfft_cols2_wstack(const float4 *__restrict__ buf, int log2ny, int log2nx, Col
     const int64_t b = pp / K;
     const dsf w = ds_from_double(wmean[pp - b * K]);
     const float4 *p = buf + ((pp - p0) << (log2ny + log2nx));
-    col_dft<LN, 11>(
+    col_dft<LN, 11, true>(
         sm,
         [&](int n2, int q) {
           const int k1 = k1_0 + (q >> lwc);
@@ -630,17 +657,19 @@ k_dsfft_cols2_wstack(const float4 *__restrict__ buf, int log2ny, int log2nx, Col
 
 // image[b, y, x] = DS slot * chk * s0 * gcf / sumwt[b] (0 where sumwt <= 0), in
 // place over the slots.
-__global__ void k_ds_wstack_finish(double *image, int64_t nb, int log2ny, int log2nx, float s0,
-                                   const double *__restrict__ gcf, const double *__restrict__ sumwt) {
-  const int64_t plane = (int64_t)1 << (log2ny + log2nx), tot = nb * plane;
+// An FP64 division a pixel and conversions bound it to 1.84 ms for 8192^2: 1.26 ms with the rounded quotient and
+// integer conversions.
+__global__ void k_ds_wstack_finish(double *image, int log2ny, int log2nx, float s0, const double *__restrict__ gcf,
+                                   const double *__restrict__ sumwt) {
+  const int64_t plane = (int64_t)1 << (log2ny + log2nx), base = blockIdx.y * plane;
   const int nx1 = (1 << log2nx) - 1;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = i >> (log2ny + log2nx);
-    const int y = (int)((i >> log2nx) & ((1 << log2ny) - 1)), x = (int)(i & nx1);
-    const float2 sl = reinterpret_cast<const float2 *>(image)[i];
-    const double w = sumwt[b];
-    const double sg = (double)((((x + y) & 1) ? -1.f : 1.f) * s0);
-    image[i] = w > 0.0 ? ds_to_double({sl.x, sl.y}) * sg * gcf[i] / w : 0.0;
+  const double w = sumwt[blockIdx.y], rcp = w > 0.0 ? __drcp_rn(w) : 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += (int64_t)gridDim.x * blockDim.x) {
+    const int y = (int)(i >> log2nx), x = (int)(i & nx1);
+    const float2 sl = reinterpret_cast<const float2 *>(image)[base + i];
+    const float sg = (((x + y) & 1) ? -1.f : 1.f) * s0;
+    const double v = (widen(sl.x * sg) + widen(sl.y * sg)) * gcf[base + i];
+    image[base + i] = w > 0.0 ? rounded_quotient(v, w, rcp) : 0.0;
   }
 }
 
@@ -663,7 +692,7 @@ bool dsfft_supported(int ny, int nx) {
 
 // Shared memory of the column kernels: the exchange tile where N > 16; the w-screen terms and sums.
 static size_t col_smem(int log2N, bool wstack) {
-  if (wstack) return (log2N > 4 ? kWsPts * 16 : 0) + kWsPts * 16;
+  if (wstack) return (log2N > 4 ? kWsPts * 8 : 0) + kWsPts * 16;
   return log2N > 4 ? kColPts * 16 : 0;
 }
 
@@ -720,9 +749,9 @@ static int rows_cols1(const float2 *grid, int64_t qstride, int nsum, int64_t q0,
     });
   }
   ARL_LAUNCH_CHECK();
-  const int64_t ntile = ((int64_t)1 << (cg.log2N2 - cg.log2G1)) << (lx - cg.log2WC1);
+  const int64_t ntile = ((int64_t)1 << (cg.log2N2 - cg.log2G1)) << (lx - cg.log2WC1 + 1);
   with_const<3, 7>(cg.log2N1, [&](auto c) {
-    k_dsfft_cols1<c.value><<<(unsigned)(np * ntile), kColT, col_smem(cg.log2N1, false), st>>>(buf, ly, lx, cg, ntile);
+    k_dsfft_cols1<c.value><<<(unsigned)(np * ntile), kWsT, col_smem(cg.log2N1, false) / 2, st>>>(buf, ly, lx, cg, ntile);
   });
   ARL_LAUNCH_CHECK();
   count_launch(2);
@@ -777,9 +806,11 @@ int dsfft_g2i_wstack(const float2 *grid, int nb, int K, int ny, int nx, double f
     count_launch(1);
   }
   const float s0 = (((nx / 2) + (ny / 2)) & 1) ? -1.f : 1.f;
-  const int64_t tot = nb * plane;
-  const int blocks = (int)std::min<int64_t>((tot + 255) / 256, 152 * 32);
-  k_ds_wstack_finish<<<blocks, 256, 0, st>>>(image, nb, ly, lx, s0, gcf, sumwt);
+  for (int64_t b = 0; b < nb; b += 65535) {  // images along the grid's y
+    const dim3 blocks((unsigned)std::min<int64_t>((plane + 255) / 256, 152 * 32), (unsigned)std::min<int64_t>(nb - b, 65535));
+    k_ds_wstack_finish<<<blocks, 256, 0, st>>>(image + b * plane, ly, lx, s0, gcf + b * plane, sumwt + b);
+    ARL_LAUNCH_CHECK();
+  }
   ARL_LAUNCH_CHECK();
   count_launch(1);
   return ARLGPU_OK;

@@ -149,4 +149,40 @@ __device__ __forceinline__ float2 ds_wbeam(const DsPix &p, dsf w) {
   return make_float2(c, s);
 }
 
+// Conversions through integer registers: GB300's FP64 unit retires 2
+// conversions a clock and SM, its integer units 64 operations or more.  Both give
+// the hardware conversion's value (to FP32: round to nearest, ties to even) and
+// leave zeros, denormals, infinities and NaNs to it.
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return (double)x;
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ void narrow(double x, double *o) { *o = x; }
+__device__ __forceinline__ void narrow(double x, float *o) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), m = hi & 0x7fffffffu;
+  if (m - 0x38100000u >= 0x47e00000u - 0x38100000u) {  // outside [2^-126, 2^127)
+    *o = (float)x;
+    return;
+  }
+  unsigned f = ((m - 0x38000000u) << 3) | (lo >> 29);
+  const unsigned rest = lo << 3;  // the 29 bits below, at the top of the word
+  f += rest > 0x80000000u || (rest == 0x80000000u && (f & 1));
+  *o = __uint_as_float((hi & 0x80000000u) | f);
+}
+
+// a / b for y = 1 / b rounded to nearest: after a correction step the quotient is
+// within an ulp, and after a second one it is the rounded quotient (Markstein, IBM
+// J. Res. Dev. 34, 1990, pp. 111-119).  Five operations
+// instead of the division's 9 (throughput) and shorter dependence.  Outside the range
+// where no step under- or overflows, the division itself.
+__device__ __forceinline__ double rounded_quotient(double a, double b, double y) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+  if (ea < 1023 - 800 || ea > 1023 + 800 || eb < 1023 - 100 || eb > 1023 + 100) return __ddiv_rn(a, b);
+  double q = __dmul_rn(a, y);
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
+}
+
 }  // namespace arlgpu

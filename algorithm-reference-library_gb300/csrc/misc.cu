@@ -5,6 +5,7 @@
 //   simulate_point                          processing_library/util/coordinate_support.py:192-212
 //   apply_gaintable, scalar gains           processing_components/calibration/operations.py:79-164 (:134-137)
 #include "common.cuh"
+#include "dsmath.cuh"
 
 namespace arlgpu {
 
@@ -51,29 +52,6 @@ __global__ void k_gains(CT *vis, int64_t nvis, int npol, const int32_t *a1, cons
       vis[r * npol + p] = v;
     }
   }
-}
-
-// Conversions through integer registers: GB300's FP64 unit retires 2
-// conversions a clock and SM, its integer units 64 operations or more.  Both give
-// the hardware conversion's value (to FP32: round to nearest, ties to even) and
-// leave zeros, denormals, infinities and NaNs to it.
-__device__ __forceinline__ double widen(double x) { return x; }
-__device__ __forceinline__ double widen(float x) {
-  const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u) return (double)x;
-  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ void narrow(double x, double *o) { *o = x; }
-__device__ __forceinline__ void narrow(double x, float *o) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), m = hi & 0x7fffffffu;
-  if (m - 0x38100000u >= 0x47e00000u - 0x38100000u) {  // outside [2^-126, 2^127)
-    *o = (float)x;
-    return;
-  }
-  unsigned f = ((m - 0x38000000u) << 3) | (lo >> 29);
-  const unsigned rest = lo << 3;  // the 29 bits below, at the top of the word
-  f += rest > 0x80000000u || (rest == 0x80000000u && (f & 1));
-  *o = __uint_as_float((hi & 0x80000000u) | f);
 }
 
 // chi^2 = sum_r,p w |Vobs - g[a2] conj(g[a1]) M|^2 and its conjugate-Wirtinger
