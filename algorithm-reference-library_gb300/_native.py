@@ -62,6 +62,8 @@ SIGNATURES = {
     'arlgpu_convert_blocks': (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_int, _vp,
                                              _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     'arlgpu_decoalesce': (ctypes.c_int, [_vp, _i64, _vp, _i32, _i32, _i32, _i32, ctypes.c_int, _vp, _vp, _vp]),
+    'arlgpu_unpack_rows': (ctypes.c_int, [_vp, _i64, _i64, _i32, _i32, _i32, _i32, _i32, ctypes.c_int, _vp, _vp, _vp,
+                                          _vp, _vp]),
     'arlgpu_dft_predict': (ctypes.c_int, [_vp, _vp, _i64, _vp, _vp, _i32, _i32, _i32, ctypes.c_int, _vp, _vp]),
     'arlgpu_row_channels_bytes': (ctypes.c_int, [_i32, _P(_sz)]),
     'arlgpu_row_channels': (ctypes.c_int, [_vp, _i64, _i32, _vp, _vp, _vp, _sz, _vp]),

@@ -97,6 +97,30 @@ static int nblk(int64_t n) {
   return (int)(b < 1 ? 1 : (b > 152 * 32 ? 152 * 32 : b));
 }
 
+// Columns of a host row table that was uploaded as it lies (one record of `stride`
+// bytes a row, every field 8-byte words): gathering strided columns on the host and
+// pinning them took 1.8 ms for 121 K rows, the records' upload and this kernel 0.15 ms.
+template <typename CT, typename W>
+__global__ void k_unpack_rows(const char *__restrict__ rec, int64_t nvis, int64_t stride, int npol, int uvw_at,
+                              int freq_at, int vis_at, int wt_at, double *__restrict__ uvw, double *__restrict__ freq,
+                              CT *__restrict__ vis, W *__restrict__ wt) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nvis; r += (int64_t)gridDim.x * blockDim.x) {
+    const char *p = rec + r * stride;
+    const double *u = reinterpret_cast<const double *>(p + uvw_at);
+    for (int d = 0; d < 3; ++d) uvw[3 * r + d] = u[d];
+    freq[r] = *reinterpret_cast<const double *>(p + freq_at);
+    if (vis)
+      for (int k = 0; k < npol; ++k) {
+        const double *v = reinterpret_cast<const double *>(p + vis_at) + 2 * k;
+        CT o;
+        o.x = v[0];
+        o.y = v[1];
+        vis[r * npol + k] = o;
+        wt[r * npol + k] = (W)reinterpret_cast<const double *>(p + wt_at)[k];
+      }
+  }
+}
+
 }  // namespace arlgpu
 
 using namespace arlgpu;
@@ -168,6 +192,33 @@ extern "C" int arlgpu_decoalesce(const void *rows, int64_t nrows, const int64_t 
     default:
       return fail(ARLGPU_ERR_INVALID, "elem_bytes must be 4, 8 or 16");
   }
+  ARL_LAUNCH_CHECK();
+  count_launch(1);
+  return ARLGPU_OK;
+}
+
+extern "C" int arlgpu_unpack_rows(const void *records, int64_t nvis, int64_t stride, int32_t npol, int32_t uvw_at,
+                                  int32_t freq_at, int32_t vis_at, int32_t weight_at, int precision, double *uvw,
+                                  double *frequency, void *vis, void *weight, void *stream) {
+  if (precision != ARLGPU_FP32C && precision != ARLGPU_FP64) return fail(ARLGPU_ERR_INVALID, "bad precision");
+  if (nvis < 0 || npol < 1 || stride < 8) return fail(ARLGPU_ERR_INVALID, "bad sizes");
+  if (nvis == 0) return ARLGPU_OK;
+  if (!records || !uvw || !frequency || !vis != !weight) return fail(ARLGPU_ERR_INVALID, "null array argument");
+  if (((uintptr_t)records | (uintptr_t)stride | uvw_at | freq_at | vis_at | weight_at) & 7)
+    return fail(ARLGPU_ERR_INVALID, "records, stride and offsets must be multiples of 8 bytes");
+  auto inside = [&](int64_t at, int64_t bytes) { return at >= 0 && at + bytes <= stride; };
+  if (!inside(uvw_at, 24) || !inside(freq_at, 8) || (vis && (!inside(vis_at, 16 * npol) || !inside(weight_at, 8 * npol))))
+    return fail(ARLGPU_ERR_INVALID, "field outside its record");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const char *rec = static_cast<const char *>(records);
+  const int64_t want = (nvis + 255) / 256;
+  const int blocks = (int)(want < 152 * 32 ? want : 152 * 32);
+  if (precision == ARLGPU_FP64)
+    k_unpack_rows<<<blocks, 256, 0, st>>>(rec, nvis, stride, npol, uvw_at, freq_at, vis_at, weight_at, uvw, frequency,
+                                          static_cast<double2 *>(vis), static_cast<double *>(weight));
+  else
+    k_unpack_rows<<<blocks, 256, 0, st>>>(rec, nvis, stride, npol, uvw_at, freq_at, vis_at, weight_at, uvw, frequency,
+                                          static_cast<float2 *>(vis), static_cast<float *>(weight));
   ARL_LAUNCH_CHECK();
   count_launch(1);
   return ARLGPU_OK;

@@ -387,6 +387,9 @@ def deconvolve_cube(dirty, psf, prefix='', **kwargs):
     residual Image).  ``psf.data`` is cropped in place, as in the reference."""
     assert isinstance(dirty, Image), dirty
     assert isinstance(psf, Image), psf
+    algorithm = get_parameter(kwargs, 'algorithm', 'msclean')
+    if algorithm in ('hogbom', 'msclean'):
+        return _deconvolve_planes(dirty, psf, algorithm, prefix, kwargs)
     dd = dirty.data.cpu().numpy() if isinstance(dirty.data, torch.Tensor) else numpy.asarray(dirty.data)
     window = clean_window(dd.shape, get_parameter(kwargs, 'window_shape', None),
                           get_parameter(kwargs, 'window_edge', 16))
@@ -394,37 +397,48 @@ def deconvolve_cube(dirty, psf, prefix='', **kwargs):
     if isinstance(mask, Image):
         window = numpy.asarray(mask.data)
     crop_psf_to_support(psf, get_parameter(kwargs, 'psf_support', max(dd.shape[2] // 2, dd.shape[3] // 2)))
-    algorithm = get_parameter(kwargs, 'algorithm', 'msclean')
     if algorithm == 'hogbom-complex':
         return _deconvolve_cube_complex(dd, psf, window, kwargs, dirty.wcs)
     if algorithm in ('msmfsclean', 'mfsmsclean', 'mmclean'):
         return _deconvolve_cube_msmfs(dirty, psf, window, kwargs)
-    if algorithm not in ('hogbom', 'msclean'):
-        raise ValueError('deconvolve_cube %s: Unknown algorithm %s' % (prefix, algorithm))
+    raise ValueError('deconvolve_cube %s: Unknown algorithm %s' % (prefix, algorithm))
+
+
+def _deconvolve_planes(dirty, psf, algorithm, prefix, kwargs):
+    """One 'hogbom' or 'msclean' per (channel, polarisation), each plane on the device
+    from its own array or tensor; the results come back into the host cubes once."""
+    device = dv.require_cuda()
+    shape = tuple(dirty.data.shape)
+    mask = get_parameter(kwargs, 'mask', None)
+    edge = get_parameter(kwargs, 'window_edge', 16)
+    window = clean_window(shape[2:], get_parameter(kwargs, 'window_shape', None), edge)
+    if window is not None:
+        window = _plane(window, device)
+    masks = mask.data if isinstance(mask, Image) else None
+    crop_psf_to_support(psf, get_parameter(kwargs, 'psf_support', max(shape[2] // 2, shape[3] // 2)))
     gain = get_parameter(kwargs, 'gain', 0.7)
     assert 0.0 < gain < 2.0, "Loop gain must be between 0 and 2"
     thresh = get_parameter(kwargs, 'threshold', 0.0)
     assert thresh >= 0.0
     niter = get_parameter(kwargs, 'niter', 100)
     assert niter > 0
-    if algorithm == 'msclean':
-        scales = get_parameter(kwargs, 'scales', [0, 3, 10, 30])
-        fracthresh = get_parameter(kwargs, 'fractional_threshold', 0.01)
-    else:
-        fracthresh = get_parameter(kwargs, 'fractional_threshold', 0.1)
+    scales = get_parameter(kwargs, 'scales', [0, 3, 10, 30])
+    fracthresh = get_parameter(kwargs, 'fractional_threshold', 0.01 if algorithm == 'msclean' else 0.1)
     assert 0.0 < fracthresh < 1.0
-    pd = psf.data.cpu().numpy() if isinstance(psf.data, torch.Tensor) else numpy.asarray(psf.data)
-    comp = numpy.zeros(dd.shape)
-    resid = numpy.zeros(dd.shape)
-    for ch in range(dd.shape[0]):
-        for pol in range(dd.shape[1]):
-            if pd[ch, pol].max():
-                w = None if window is None else window[ch, pol]
-                if algorithm == 'msclean':
-                    comp[ch, pol], resid[ch, pol] = msclean(dd[ch, pol], pd[ch, pol], w, gain, thresh, niter,
-                                                            scales, fracthresh, prefix)
-                else:
-                    comp[ch, pol], resid[ch, pol] = hogbom(dd[ch, pol], pd[ch, pol], w, gain, thresh, niter,
-                                                           fracthresh, prefix)
+    comp = numpy.zeros(shape)
+    resid = numpy.zeros(shape)
+    for ch in range(shape[0]):
+        for pol in range(shape[1]):
+            p = _plane(psf.data[ch, pol], device)
+            if not float(p.max().item()):
+                continue
+            d = _plane(dirty.data[ch, pol], device)
+            w = window if masks is None else _plane(masks[ch, pol], device)
+            if algorithm == 'msclean':
+                c, r = msclean(d, p, w, gain, thresh, niter, scales, fracthresh, prefix)
+            else:
+                c, r = hogbom(d, p, w, gain, thresh, niter, fracthresh, prefix)
+            torch.from_numpy(comp[ch, pol]).copy_(c)
+            torch.from_numpy(resid[ch, pol]).copy_(r)
     return (create_image_from_array(comp, dirty.wcs, dirty.polarisation_frame),
             create_image_from_array(resid, dirty.wcs, dirty.polarisation_frame))

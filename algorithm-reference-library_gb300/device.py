@@ -228,8 +228,45 @@ def fft_image_to_grid(image_t, gcf_t, gd, precision, out=None, stream=None):
 
 
 def to_device(a, dtype, device, non_blocking=True):
-    """Host NumPy array -> device tensor through pinned memory."""
-    t = torch.from_numpy(numpy.ascontiguousarray(a)).to(dtype)
-    if device.type == 'cuda':
-        t = t.pin_memory().to(device, non_blocking=non_blocking)
-    return t
+    """Host NumPy array -> device tensor.  Straight from the array's own pages: a
+    pinned copy first costs a pass over the data (0.35 ms for 7 MB) and the driver
+    stages pageable memory at the link's rate."""
+    return torch.from_numpy(numpy.ascontiguousarray(a)).to(dtype).to(device, non_blocking=non_blocking)
+
+
+_UNPACK_ROWS = 1 << 22
+
+
+def host_rows(vis, precision, device, need_vis=True):
+    """(uvw, frequency, vis, imaging weight) device tensors of a host Visibility
+    (the last two None without ``need_vis``).  The table goes up as it lies and its
+    columns are taken apart on the device, 2^22 rows at a time; a table that is not
+    one block of native 64-bit fields is gathered column by column on the host."""
+    data = vis.data
+    fields = {k: data.dtype.fields.get(k) for k in ('uvw', 'frequency', 'vis', 'imaging_weight')}
+    npol = data['vis'].shape[1]
+    want = {'uvw': ('f8', (3,)), 'frequency': ('f8', ()), 'vis': ('c16', (npol,)), 'imaging_weight': ('f8', (npol,))}
+    plain = (type(data) is numpy.ndarray and data.ndim == 1 and data.flags.c_contiguous and data.flags.writeable
+             and data.dtype.itemsize % 8 == 0 and data.ctypes.data % 8 == 0
+             and all(f is not None and f[0] == numpy.dtype(want[k]) and f[1] % 8 == 0 for k, f in fields.items()))
+    if not plain:
+        uvw = to_device(vis.uvw, torch.float64, device)
+        f = to_device(vis.frequency, torch.float64, device)
+        if not need_vis:
+            return uvw, f, None, None
+        return (uvw, f, to_device(vis.vis, torch.complex128, device).to(CDTYPE[precision]),
+                to_device(vis.imaging_weight, torch.float64, device).to(RDTYPE[precision]))
+    n, size = data.shape[0], data.dtype.itemsize
+    uvw = torch.empty((n, 3), dtype=torch.float64, device=device)
+    f = torch.empty(n, dtype=torch.float64, device=device)
+    v = torch.empty((n, npol), dtype=CDTYPE[precision], device=device) if need_vis else None
+    w = torch.empty((n, npol), dtype=RDTYPE[precision], device=device) if need_vis else None
+    at = [fields[k][1] for k in ('uvw', 'frequency', 'vis', 'imaging_weight')]
+    raw = torch.from_numpy(data.view(numpy.uint8))
+    for b in range(0, n, _UNPACK_ROWS):
+        e = min(b + _UNPACK_ROWS, n)
+        rec = raw[b * size:e * size].to(device)
+        nat.call('arlgpu_unpack_rows', nat.ptr(rec), e - b, size, npol, *at, nat.PRECISIONS[precision],
+                 nat.ptr(uvw[b:e]), nat.ptr(f[b:e]), nat.ptr(None if v is None else v[b:e]),
+                 nat.ptr(None if w is None else w[b:e]), nat.stream_ptr())
+    return uvw, f, v, w

@@ -55,11 +55,7 @@ class DeviceVisibility:
     def from_visibility(cls, vis, precision=None, device=None):
         precision = dv.resolve_precision(precision)
         device = device or dv.require_cuda()
-        return cls(dv.to_device(vis.uvw, torch.float64, device),
-                   dv.to_device(vis.frequency, torch.float64, device),
-                   dv.to_device(vis.vis, torch.complex128, device).to(dv.CDTYPE[precision]),
-                   dv.to_device(vis.imaging_weight, torch.float64, device).to(dv.RDTYPE[precision]),
-                   vis.polarisation_frame, vis.phasecentre)
+        return cls(*dv.host_rows(vis, precision, device), vis.polarisation_frame, vis.phasecentre)
 
 
 def _rows(vis, precision, device, need_vis=True):
@@ -68,13 +64,7 @@ def _rows(vis, precision, device, need_vis=True):
         w = vis.imaging_weight.to(dv.RDTYPE[precision]) if need_vis else None
         return vis.uvw, vis.frequency, v, w
     assert isinstance(vis, Visibility), vis
-    uvw = dv.to_device(vis.uvw, torch.float64, device)
-    f = dv.to_device(vis.frequency, torch.float64, device)
-    if not need_vis:
-        return uvw, f, None, None
-    v = dv.to_device(vis.vis, torch.complex128, device).to(dv.CDTYPE[precision])
-    w = dv.to_device(vis.imaging_weight, torch.float64, device).to(dv.RDTYPE[precision])
-    return uvw, f, v, w
+    return dv.host_rows(vis, precision, device, need_vis)
 
 
 def _descs(griddata, cf, precision, device):

@@ -294,6 +294,15 @@ int arlgpu_decoalesce(const void *rows, int64_t nrows, const int64_t *cindex, in
                       int32_t nchan, int32_t npol, int elem_bytes, void *block, int64_t *n_bad_dev,
                       void *stream);
 
+/* Columns of a Visibility table (memory_data_models.py:745-937) uploaded as it lies: nvis
+ * records of `stride` bytes (device), with uvw (3 float64), frequency (float64), vis (npol
+ * complex128) and imaging weight (npol float64) at the given byte offsets, all multiples of
+ * 8.  Writes uvw [nvis][3], frequency [nvis] and, unless vis and weight are NULL, vis and
+ * weight [nvis][npol] in the precision's types. */
+int arlgpu_unpack_rows(const void *records, int64_t nvis, int64_t stride, int32_t npol, int32_t uvw_at,
+                       int32_t freq_at, int32_t vis_at, int32_t weight_at, int precision, double *uvw,
+                       double *frequency, void *vis, void *weight, void *stream);
+
 /* ---- (f3) DFT predict: predict_skycomponent_visibility (imaging/base.py:192-244) with
  * simulate_point (util/coordinate_support.py:192-212) ----
  * arlgpu_dft_predict: vis[r][p] += sum_k flux[k][row_chan[r]][p] exp(-2 pi i (u l + v m + w n))
