@@ -102,7 +102,7 @@ struct Geom {
   uint32_t nbins;  // nchan * nw * ntv * ntu; key == nbins marks a rejected row
 };
 
-int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precision, Geom *g);
+int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precision, int64_t nvis, Geom *g);
 
 // Workspace carve-up for a plan over nvis rows.
 struct PlanBufs {

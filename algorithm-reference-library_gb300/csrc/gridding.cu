@@ -1689,6 +1689,281 @@ __device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsign
   return d;
 }
 
+// K3 (one warp per tile; small supports without per-plane ones).
+//
+// A CTA is one warp with a subgrid of its own, so a row's taps are added by plain
+// shared-memory reads and writes: no atomics, no barriers, and no pass over the
+// segment's rows before the first is added.  FP32C cells hold (sum, compensation) of
+// both parts as one float4 and a tap adds by Knuth's TwoSum; FP64 cells hold the
+// sums, added by FMAs (an FP64 shared atomic is a compare-and-swap loop), two of the
+// four left out for a row whose taps are all real, as a PSWF's are.  The window's
+// S^2 taps are consecutive in the table, so lane l takes taps l, l + 32, ...: its
+// cells' offsets in the window are constants, and eight lanes cover one row of an
+// 8-wide window, which is conflict-free.  Rows are prepared 32 at a time, one per
+// lane (the next 32 rows' maps and values are loaded meanwhile), and the taps of
+// some rows are in flight while others are added.
+//
+// What bounds it is shared-memory bandwidth in FP32C (16 bytes read, 16 written
+// and 8 bytes of tap per tap and lane) and the FP64 unit in FP64, once enough warps
+// are resident: each owns S_G^2 cells of 16 bytes a polarisation, so the subgrid is
+// small (make_geom).  Measured against the CTA-wide kernels (k_grid_fx with its
+// row copy, k_grid_lean), us:
+//   FP32C, 1 pol, 8 M rows, S = 8, O = 8       1174 -> 987   (subgrid 48 -> 32)
+//   FP32C, 1 pol, 15.6 M rows (gain solve)     2157 -> 1717
+//   FP32C, 1 pol, S = 10 (four taps a lane)    1413 -> 1514: not taken
+//   FP32C, 2 or 4 pols, S = 8                  555 -> 694, 817 -> 1881: not taken
+//   FP32C, 1 pol, 25 M rows, 32 slices         6229 -> 3588
+//   FP64, 1 pol, 1.95 M rows, S = 8 / 10       1921 -> 958, 3335 -> 1810
+//   FP64, 2 pols, 1.95 M rows, S = 8 / 10      3735 -> 1886, 6570 -> 3549
+//   FP64, 1 pol, S = 12                        1136 -> 1236: not taken
+template <typename R> struct OwnCell;
+__device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ bool finite_bits(float x) { return (__float_as_int(x) & 0x7f800000) != 0x7f800000; }
+template <> struct OwnCell<float> {
+  using T = float4;
+  __device__ static __forceinline__ float4 add(float4 o, float2 t, float2 v) {
+    // conj(t) v, then TwoSum on (re, im) pairs
+    const float2 c = make_float2(t.x * v.x + t.y * v.y, t.x * v.y - t.y * v.x);
+    const float2 s = make_float2(__fadd_rn(o.x, c.x), __fadd_rn(o.y, c.y));
+    const float2 b = make_float2(__fsub_rn(s.x, o.x), __fsub_rn(s.y, o.y));
+    const float ex = __fadd_rn(__fsub_rn(o.x, __fsub_rn(s.x, b.x)), __fsub_rn(c.x, b.x));
+    const float ey = __fadd_rn(__fsub_rn(o.y, __fsub_rn(s.y, b.y)), __fsub_rn(c.y, b.y));
+    return make_float4(s.x, s.y, __fadd_rn(o.z, ex), __fadd_rn(o.w, ey));
+  }
+  __device__ static __forceinline__ float4 add_real(float4 o, float2 t, float2 v) { return add(o, t, v); }
+  __device__ static __forceinline__ float2 value(float4 o) { return make_float2(o.x + o.z, o.y + o.w); }
+  __device__ static __forceinline__ float4 zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+};
+template <> struct OwnCell<double> {
+  using T = double2;
+  __device__ static __forceinline__ double2 add(double2 o, double2 t, double2 v) {
+    return make_double2(fma(t.x, v.x, fma(t.y, v.y, o.x)), fma(t.x, v.y, fma(-t.y, v.x, o.y)));
+  }
+  __device__ static __forceinline__ double2 add_real(double2 o, double2 t, double2 v) {
+    return make_double2(fma(t.x, v.x, o.x), fma(t.x, v.y, o.y));
+  }
+  __device__ static __forceinline__ double2 value(double2 o) { return o; }
+  __device__ static __forceinline__ double2 zero() { return make_double2(0.0, 0.0); }
+};
+
+// One row as the lanes read it back: the offsets of its kernel (elements) and of its
+// window in the subgrid (cells), and vis * weight.
+template <typename R, int NPOL> struct alignas(16) OwnRow {
+  int koff, cell;
+  typename Cplx<R>::T vw[NPOL];
+};
+
+template <typename R, int NPOL, int STEPS>
+__global__ void __launch_bounds__(32)
+k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__ sidx,
+           const uint32_t *__restrict__ off, uint32_t chunk, const typename Cplx<R>::T *__restrict__ vis,
+           const typename VisT<R>::W *__restrict__ wt, const typename Cplx<R>::T *__restrict__ cf,
+           typename Cplx<R>::T *__restrict__ grid, double *__restrict__ sumwt, uint32_t *__restrict__ queue) {
+  using CT = typename Cplx<R>::T;
+  using Cell = typename OwnCell<R>::T;
+  using Row = OwnRow<R, NPOL>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(16) Row s_row[32];
+  Cell *sub = reinterpret_cast<Cell *>(smraw);  // [NPOL][SG][SG], zero between segments
+  const int lane = threadIdx.x, S = g.S, SG = g.SG, SG2 = SG * SG, n = S * S, ps = (int)g.cf_pol_stride;
+  const uint32_t nvalid = off[g.nbins];
+  for (int k = lane; k < NPOL * SG2; k += 32) sub[k] = OwnCell<R>::zero();
+  int cofs[STEPS];  // this lane's cells in the window; -1: no tap
+#pragma unroll
+  for (int u = 0; u < STEPS; ++u) {
+    const int t = lane + 32 * u;
+    cofs[u] = t < n ? t / S * SG + t % S : -1;
+  }
+  const int64_t plane_elems = (int64_t)g.ny * g.nx;
+  uint64_t cb = blockIdx.x;
+  while (cb * chunk < nvalid) {
+    const uint32_t c0 = (uint32_t)(cb * chunk), c1 = min(c0 + chunk, nvalid);
+    uint32_t pos = c0;
+    while (pos < c1) {
+      const SegInfo sg = seg_at(pos, c1, smap, off, g);
+      CT *tile = grid + ((int64_t)sg.ch * NPOL * g.nw + sg.zg) * plane_elems;
+      double wsum[NPOL];
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) wsum[p] = 0.0;
+      float wf[NPOL], we[NPOL];  // FP32C: the weights' sum and its TwoSum error
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) wf[p] = we[p] = 0.f;
+      int x0 = 0x7fffffff, y0 = 0x7fffffff, x1 = -1, y1 = -1;
+      // rows of the next batch, loaded ahead
+      RowMap m{};
+      uint32_t idx = 0;
+      CT v[NPOL];
+      R w[NPOL];
+      auto load_map = [&](uint32_t r) {
+        if (r < sg.end) {
+          m = smap[r];
+          idx = sidx[r];
+        }
+      };
+      auto load_val = [&](uint32_t r) {
+#pragma unroll
+        for (int p = 0; p < NPOL; ++p) {
+          v[p] = czero<CT>();
+          w[p] = (R)0;
+          if (r < sg.end) {
+            v[p] = vis[(size_t)idx * NPOL + p];
+            w[p] = wt[(size_t)idx * NPOL + p];
+          }
+        }
+      };
+      load_map(pos + lane);
+      load_val(pos + lane);
+      for (uint32_t b0 = pos; b0 < sg.end; b0 += 32) {
+        const int cnt = (int)min(32u, sg.end - b0);
+        __syncwarp();
+        if (lane < cnt) {
+          const int lx = m.pu - (S >> 1) - sg.u0, ly = m.pv - (S >> 1) - sg.v0;
+          const int uf = m.sub & 0xff, vf = (m.sub >> 8) & 0xff, zc = m.sub >> 16;
+          x0 = min(x0, lx), x1 = max(x1, lx), y0 = min(y0, ly), y1 = max(y1, ly);
+          Row &o = s_row[lane];
+          o.koff = (int)(sg.ch * g.cf_chan_stride + zc * g.cf_z_stride) + (vf * g.O + uf) * n;
+          o.cell = ly * SG + lx;
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) {
+            o.vw[p].x = v[p].x * w[p];
+            o.vw[p].y = v[p].y * w[p];
+            if constexpr (sizeof(R) == 4) {
+              const float s2 = wf[p] + w[p], bp = s2 - wf[p];
+              we[p] += (wf[p] - (s2 - bp)) + (w[p] - bp);
+              wf[p] = s2;
+            } else {
+              wsum[p] += w[p];
+            }
+          }
+        }
+        __syncwarp();
+        load_map(b0 + 32 + lane);
+        if (sg.direct) {
+          load_val(b0 + 32 + lane);
+          for (int i = 0; i < cnt; ++i) {
+            const Row rw = s_row[i];
+            const CT *k = cf + rw.koff + lane;
+            const int cy = rw.cell / SG, cx = rw.cell - cy * SG;
+            CT *o = tile + (int64_t)(sg.v0 + cy) * g.nx + sg.u0 + cx;
+#pragma unroll
+            for (int u = 0; u < STEPS; ++u) {
+              if (cofs[u] < 0) continue;
+              const int t = lane + 32 * u, ty = t / S;
+#pragma unroll
+              for (int p = 0; p < NPOL; ++p) {
+                const CT tp = k[p * ps + 32 * u];
+                CT c;
+                c.x = tp.x * rw.vw[p].x + tp.y * rw.vw[p].y;
+                c.y = tp.x * rw.vw[p].y - tp.y * rw.vw[p].x;
+                red_global<CT>(o + (int64_t)p * g.nw * plane_elems + (int64_t)ty * g.nx + (t - ty * S), c);
+              }
+            }
+          }
+          continue;
+        }
+        // Taps of GR rows at a time.  With one kernel for every polarisation (pol stride 0, as
+        // ARL's PSWF and w-kernels are) a tap is loaded once, else the polarisations take turns.
+        constexpr int GR = STEPS <= 2 ? 4 : 2;
+        auto load = [&](int i0, int p, CT(&tp)[GR][STEPS], Row(&rec)[GR]) {
+#pragma unroll
+          for (int r = 0; r < GR; ++r) {
+            const Row &rw = s_row[min(i0 + r, cnt - 1)];
+            if (sizeof(R) == 4) rec[r] = rw;
+            const CT *k = cf + rw.koff + p * ps + lane;
+#pragma unroll
+            for (int u = 0; u < STEPS; ++u) tp[r][u] = cofs[u] >= 0 ? k[32 * u] : czero<CT>();
+          }
+        };
+        auto add = [&](int i0, int p0, int p1, CT(&tp)[GR][STEPS], Row(&rec)[GR]) {
+#pragma unroll
+          for (int r = 0; r < GR; ++r) {
+            if (i0 + r >= cnt) break;
+            __syncwarp();  // the row before has added to other lanes' cells
+            const Row &rw = sizeof(R) == 4 ? rec[r] : s_row[i0 + r];
+            bool real = false;  // FP64: every tap of the row real
+            if constexpr (sizeof(R) == 8) {
+              real = true;
+#pragma unroll
+              for (int u = 0; u < STEPS; ++u) real = real && (__double_as_longlong(tp[r][u].y) << 1) == 0;
+              real = __all_sync(0xffffffffu, real);
+            }
+#pragma unroll
+            for (int p = 0; p < NPOL; ++p) {
+              if (p < p0 || p >= p1) continue;
+              Cell *c = sub + p * SG2 + rw.cell;
+              const CT vw = rw.vw[p];
+              // a zero tap times an infinity or NaN is a NaN: such rows take the whole product
+              const bool rl = real && finite_bits(vw.x) && finite_bits(vw.y);
+              Cell o[STEPS];
+#pragma unroll
+              for (int u = 0; u < STEPS; ++u)
+                if (cofs[u] >= 0) o[u] = c[cofs[u]];
+#pragma unroll
+              for (int u = 0; u < STEPS; ++u)
+                if (cofs[u] >= 0)
+                  c[cofs[u]] = rl ? OwnCell<R>::add_real(o[u], tp[r][u], vw) : OwnCell<R>::add(o[u], tp[r][u], vw);
+            }
+          }
+        };
+        auto rows = [&](int p0, int p1) {
+          CT ta[GR][STEPS], tb[GR][STEPS];
+          Row ra[GR], rb[GR];
+          load(0, p0, ta, ra);
+          for (int i = 0; i < cnt; i += 2 * GR) {
+            if (i + GR < cnt) load(i + GR, p0, tb, rb);
+            add(i, p0, p1, ta, ra);
+            if (i == 0 && p0 == 0) load_val(b0 + 32 + lane);  // its index has arrived
+            if (i + 2 * GR < cnt) load(i + 2 * GR, p0, ta, ra);
+            if (i + GR < cnt) add(i + GR, p0, p1, tb, rb);
+          }
+        };
+        if (NPOL == 1 || ps == 0)
+          rows(0, NPOL);
+        else
+#pragma unroll 1
+          for (int p = 0; p < NPOL; ++p) rows(p, p + 1);
+      }
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) {
+        if constexpr (sizeof(R) == 4) wsum[p] = (double)wf[p] + (double)we[p];
+        for (int o = 16; o > 0; o >>= 1) wsum[p] += __shfl_xor_sync(0xffffffffu, wsum[p], o);
+        if (lane == 0 && wsum[p] != 0.0) atomicAdd(&sumwt[sg.ch * NPOL + p], wsum[p]);
+      }
+      if (!sg.direct) {
+        // Flush the footprint and clear it.
+        __syncwarp();
+        x0 = __reduce_min_sync(0xffffffffu, x0);
+        y0 = __reduce_min_sync(0xffffffffu, y0);
+        x1 = __reduce_max_sync(0xffffffffu, x1) + S;
+        y1 = __reduce_max_sync(0xffffffffu, y1) + S;
+        for (int y = y0; y < y1; ++y) {
+          const int gy = sg.v0 + y;
+          for (int x = x0 + lane; x < x1; x += 32) {
+            const int gx = sg.u0 + x;
+#pragma unroll
+            for (int p = 0; p < NPOL; ++p) {
+              Cell *c = sub + p * SG2 + y * SG + x;
+              const CT val = OwnCell<R>::value(*c);
+              *c = OwnCell<R>::zero();
+              if ((val.x == (R)0 && val.y == (R)0) || gy < 0 || gy >= g.ny || gx < 0 || gx >= g.nx) continue;
+              red_global<CT>(tile + (int64_t)p * g.nw * plane_elems + (int64_t)gy * g.nx + gx, val);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      pos = sg.end;
+    }
+    if (queue) {
+      uint32_t nx = 0;
+      if (lane == 0) nx = gridDim.x + atomicAdd(queue, 1u);
+      cb = __shfl_sync(0xffffffffu, nx, 0);
+    } else {
+      cb += gridDim.x;
+    }
+  }
+}
+
 // K4 (lean variant): warp per row, specialised on the polarisation count, tap
 // walk through the row table, groups of up to four steps in flight.
 // DUP (FP32 only, degrid_kernel 3): the staged subgrid holds each cell as
@@ -2390,7 +2665,10 @@ k_degrid_tma(const __grid_constant__ TmaDesc tmd, Geom g, const RowMap *__restri
 // ---------------------------------------------------------------------------
 static double rcp(double x) { return 1.0 / x; }
 
-int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precision, Geom *g) {
+// Rows from which a plan of one polarisation and S <= 8 has 32-cell subgrids.
+constexpr int64_t kSmallTileRows = 2 << 20;
+
+int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precision, int64_t nvis, Geom *g) {
   if (!gd || !cd) return fail(ARLGPU_ERR_INVALID, "null descriptor");
   if (precision != ARLGPU_FP32C && precision != ARLGPU_FP64)
     return fail(ARLGPU_ERR_INVALID, "precision must be ARLGPU_FP32C or ARLGPU_FP64");
@@ -2527,12 +2805,32 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
   // words) fit in 64 KiB of shared memory, else 32.
   const size_t cell = precision == ARLGPU_FP64 ? 16 : 16;  // c128, or c64 sum + c64 comp
   int SG = g_tune_subgrid.load();
-  if (SG <= 0) {
+  auto fitted = [&](int e) {
+    if (e - g->S < 8) e = ((g->S + 8 + 7) / 8) * 8;
+    return (e + 7) & ~7;  // a multiple of the band-owner warp count
+  };
+  auto bins = [&](int e) {
+    const int T = e - g->S;
+    return (uint64_t)g->nchan * g->nw * ((g->ny + T - 1) / T) * ((g->nx + T - 1) / T);
+  };
+  const bool chosen = SG > 0;
+  if (!chosen) {
     SG = 48;  // the C2 autotuning optimum for supports 8..32
     if ((size_t)g->npol * SG * SG * cell > 64 * 1024) SG = 32;
   }
-  if (SG - g->S < 8) SG = ((g->S + 8 + 7) / 8) * 8;
-  SG = (SG + 7) & ~7;  // a multiple of the band-owner warp count
+  SG = fitted(SG);
+  // Many rows of one polarisation and one small support: the one-warp gridder wants
+  // many subgrids resident (14 of 32^2 cells an SM against 6 of 48^2).  24 cells, with
+  // 24 resident, grid a little faster, but the degridder, which stages a bin's subgrid,
+  // loses where a bin has few rows.  Nor is it for fewer rows (k_grid_own), or for more
+  // tiles than rows, which would cost the plan more to scan than its rows.  S = 8, us,
+  // subgrid 48 / 32 / 24: grid 2157 / 1717 / 1539 and degrid 1569 / 1491 / 1563 (15.6 M
+  // rows of the gain solve), grid 6229 / 3588 / 3602 (25 M rows, 8192^2, 32 slices),
+  // degrid 1664 / 1655 / 2144 (12.6 M rows, 4096^2, 20 slices), 2.2 M rows spread over
+  // 1800^2 pixels grid 355 / 280 / 279, degrid 257 / 247 / 278.
+  if (!chosen && g->npol == 1 && g->S <= 8 && !g->plane_support && nvis >= kSmallTileRows &&
+      bins(fitted(32)) <= (uint64_t)nvis)
+    SG = fitted(32);
   if ((size_t)g->npol * SG * fx_pitch(SG) * cell > 200 * 1024)
     return fail(ARLGPU_ERR_UNSUPPORTED, "support %d with %d polarisations needs more shared memory than a CTA has",
                 g->S, g->npol);
@@ -2541,7 +2839,7 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
   g->rcpT = (uint32_t)(((1ull << 32) + g->T - 1) / g->T);
   g->ntu = (g->nx + g->T - 1) / g->T;
   g->ntv = (g->ny + g->T - 1) / g->T;
-  uint64_t nb = (uint64_t)g->nchan * g->nw * g->ntv * g->ntu;
+  const uint64_t nb = bins(SG);
   if (nb >= 0x7fffffffull) return fail(ARLGPU_ERR_UNSUPPORTED, "too many bins");
   g->nbins = (uint32_t)nb;
   return ARLGPU_OK;
@@ -2768,6 +3066,55 @@ static int launch_grid_fx(const Geom &g, const PlanBufs &b, int64_t nvis, const 
   return ARLGPU_OK;
 }
 
+// Whether the one-warp gridder takes a call (its comment has both sides measured):
+// rows of one support in a cf table addressable in 32 bits, FP32C with one
+// polarisation, S <= 8, the small subgrid and rows enough that their chunks give
+// every warp some (at 1 M rows 156 -> 123 us with 24 cells, at 0.1 M 53 -> 69),
+// FP64 with one or two, S <= 10 and subgrids of at most 36 KiB: six warps an SM (two
+// polarisations with 72 KiB, a subgrid edge of 48 asked for: 2021 -> 2587 us).
+static bool takes_own(const Geom &g, int64_t nvis, bool fp64) {
+  if (g.plane_support || cf_elems(g) >= 0x7fffffffll) return false;
+  return fp64 ? g.npol <= 2 && g.S <= 10 && g.npol * g.SG * g.SG <= 48 * 48
+              : g.npol == 1 && g.S <= 8 && g.SG <= 32 && nvis >= kSmallTileRows;
+}
+
+template <typename R>
+static int launch_grid_own(const Geom &g, const PlanBufs &b, int64_t nvis, const void *vis, const void *wt,
+                           const void *cf, void *grid, double *sumwt, cudaStream_t st) {
+  using CT = typename Cplx<R>::T;
+  const size_t smem = (size_t)g.npol * g.SG * g.SG * 16;
+  const bool two = g.S <= 8;  // taps a lane: two, or four
+  auto kern = k_grid_own<R, 1, 2>;
+  if constexpr (sizeof(R) == 8)
+    kern = g.npol == 1 ? (two ? k_grid_own<R, 1, 2> : k_grid_own<R, 1, 4>)
+                       : (two ? k_grid_own<R, 2, 2> : k_grid_own<R, 2, 4>);
+  ARL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int occ = 0;
+  ARL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32, smem));
+  if (occ < 1) return fail(ARLGPU_ERR_UNSUPPORTED, "gridder needs %zu bytes of shared memory", smem);
+  // Eight chunks a warp, so that the last ones to finish weigh little (with two a
+  // warp 2 M rows took 13 % longer), but no shorter than 64 rows: a bin cut by a
+  // chunk's end is flushed once more.  In FP32C a flush rounds the grid's cells to 24
+  // bits, so its chunks have 384 rows and more: the grid's RMS error is then no larger
+  // than k_grid_fx's with 512 rows of a tile of 40^2 pixels (with 256 it was 2.5e-6 of
+  // the grid's RMS against 2.2e-6 at 8 M rows, with 64 twice as large).
+  const int64_t resident = (int64_t)occ * num_sms();
+  uint32_t chunk = sizeof(R) == 8 ? 64 : 384;
+  while (chunk < chunk_rows() && nvis / (2 * (int64_t)chunk) >= 8 * resident) chunk *= 2;
+  chunk = std::min(chunk, chunk_rows());
+  const int64_t nchunks = (nvis + chunk - 1) / chunk;
+  if (nchunks <= 0) return ARLGPU_OK;
+  const unsigned blocks = (unsigned)std::min<int64_t>(nchunks, resident);
+  uint32_t *queue = work_queue(b, 0, st);
+  if (queue) ARL_CUDA(cudaMemsetAsync(queue, 0, 4, st));
+  kern<<<blocks, 32, smem, st>>>(g, b.smap, b.sidx, b.offsets, chunk, static_cast<const CT *>(vis),
+                                 static_cast<const typename VisT<R>::W *>(wt), static_cast<const CT *>(cf),
+                                 static_cast<CT *>(grid), sumwt, queue);
+  ARL_LAUNCH_CHECK();
+  count_launch(1);
+  return ARLGPU_OK;
+}
+
 template <typename R>
 static int launch_grid(const Geom &g, const PlanBufs &b, int64_t nvis, const void *vis, const void *wt,
                        const void *cf, void *grid, double *sumwt, cudaStream_t st) {
@@ -2788,6 +3135,8 @@ static int launch_grid(const Geom &g, const PlanBufs &b, int64_t nvis, const voi
     smem = (size_t)g.npol * g.SG * g.SG * sizeof(typename Cplx<R>::T) + tap_table_bytes(g.S);
   } else if (g_tune_grid_kernel.load() >= 4) {
     if (g.npol == 3) return fail(ARLGPU_ERR_UNSUPPORTED, "the lean gridder handles 1, 2 or 4 polarisations");
+    if (g_tune_grid_kernel.load() == 4 && takes_own(g, nvis, sizeof(R) == 8))
+      return launch_grid_own<R>(g, b, nvis, vis, wt, cf, grid, sumwt, st);
     if (sizeof(R) == 4 && g.tap_absmax > 0.f)
       return launch_grid_fx(g, b, nvis, vis, wt, cf, grid, sumwt, g_tune_grid_kernel.load() == 4, st);
     // FP64, or no tap bound: the compensated float variant
@@ -2897,7 +3246,6 @@ static int launch_degrid_tma(const Geom &g, const PlanBufs &b, int64_t nvis, con
                                           static_cast<float2 *>(vis_out), queue, b.queue + 2);
   ARL_LAUNCH_CHECK();
   count_launch(1);
-  *launched = true;
   return ARLGPU_OK;
 }
 
@@ -2991,7 +3339,7 @@ extern "C" int arlgpu_convolution_mapping(const double *uvw, const double *frequ
                                           int32_t *pu_off, int32_t *pv, int32_t *pv_off, int32_t *pwg,
                                           int32_t *pwc, int32_t *pfreq, int64_t *n_bad_host, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, ARLGPU_FP64, &g));
+  ARL_TRY(make_geom(gd, cd, ARLGPU_FP64, nvis, &g));
   ARL_TRY(check_rows(nvis));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   unsigned long long *d_bad = nullptr;
@@ -3013,7 +3361,7 @@ extern "C" int arlgpu_convolution_mapping(const double *uvw, const double *frequ
 extern "C" int arlgpu_plan_workspace_bytes(int64_t nvis, const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd,
                                            size_t *bytes_host) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, &g));
+  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (!bytes_host) return fail(ARLGPU_ERR_INVALID, "null bytes_host");
   *bytes_host = plan_bytes(nvis, g);
@@ -3024,7 +3372,7 @@ extern "C" int arlgpu_plan_build(const double *uvw, const double *frequency, int
                                  const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, void *workspace,
                                  size_t workspace_bytes, int64_t *n_bad_dev, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, &g));
+  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (nvis > 0 && (!uvw || !frequency)) return fail(ARLGPU_ERR_INVALID, "null uvw / frequency");
   PlanBufs b;
@@ -3036,7 +3384,7 @@ extern "C" int arlgpu_grid_planned(const void *vis, const void *weight, int64_t 
                                    const arlgpu_cf_desc *cd, void *grid, const arlgpu_grid_desc *gd, double *sumwt,
                                    const void *workspace, size_t workspace_bytes, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, precision, &g));
+  ARL_TRY(make_geom(gd, cd, precision, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (!grid || !sumwt || !cf || (nvis > 0 && (!vis || !weight))) return fail(ARLGPU_ERR_INVALID, "null array argument");
   PlanBufs b;
@@ -3053,7 +3401,7 @@ extern "C" int arlgpu_degrid_planned(int64_t nvis, int precision, const void *cf
                                      const void *grid, const arlgpu_grid_desc *gd, void *vis_out,
                                      const void *workspace, size_t workspace_bytes, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, precision, &g));
+  ARL_TRY(make_geom(gd, cd, precision, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (!grid || !cf || (nvis > 0 && !vis_out)) return fail(ARLGPU_ERR_INVALID, "null array argument");
   PlanBufs b;
@@ -3084,7 +3432,7 @@ extern "C" int arlgpu_plan_plane_mean_w(const double *uvw, int64_t nvis, const a
                                         const arlgpu_cf_desc *cd, void *workspace, size_t workspace_bytes,
                                         double *wmean, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, &g));
+  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (!wmean || (nvis > 0 && !uvw)) return fail(ARLGPU_ERR_INVALID, "null array argument");
   PlanBufs b;
@@ -3102,7 +3450,7 @@ extern "C" int arlgpu_plan_plane_mean_w(const double *uvw, int64_t nvis, const a
 extern "C" int arlgpu_plan_flags(int64_t nvis, const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd,
                                  const void *workspace, size_t workspace_bytes, uint32_t *flags_host, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, &g));
+  ARL_TRY(make_geom(gd, cd, ARLGPU_FP32C, nvis, &g));
   ARL_TRY(check_rows(nvis));
   if (!flags_host) return fail(ARLGPU_ERR_INVALID, "null flags_host");
   PlanBufs b;

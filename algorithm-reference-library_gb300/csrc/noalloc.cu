@@ -82,7 +82,7 @@ extern "C" int arlgpu_grid_noalloc(const double *uvw, const double *frequency, c
                 "arlgpu_grid_noalloc takes at most %lld rows per call (got %lld); use arlgpu_grid with a workspace",
                 (long long)kMaxRows, (long long)nvis);
   Geom g;
-  ARL_TRY(make_geom(gd, cd, precision, &g));
+  ARL_TRY(make_geom(gd, cd, precision, nvis, &g));
   if ((int64_t)g.nbins > kMaxBins)
     return fail(ARLGPU_ERR_WORKSPACE,
                 "arlgpu_grid_noalloc takes a plan of at most %lld bins per call (this grid has %u channel x "

@@ -188,7 +188,7 @@ extern "C" int arlgpu_grid_weights(const double *uvw, const double *frequency, c
                                    int precision, const arlgpu_cf_desc *cd, double *wgrid, const arlgpu_grid_desc *gd,
                                    double *sumwt, int64_t *n_bad_dev, void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, precision, &g));
+  ARL_TRY(make_geom(gd, cd, precision, nvis, &g));
   if (nvis < 0) return fail(ARLGPU_ERR_INVALID, "nvis < 0");
   if (!wgrid || !sumwt || !n_bad_dev || (nvis > 0 && (!uvw || !frequency || !weight)))
     return fail(ARLGPU_ERR_INVALID, "null array argument");
@@ -217,7 +217,7 @@ extern "C" int arlgpu_reweight(const double *uvw, const double *frequency, void 
                                const arlgpu_cf_desc *cd, const double *wgrid, const arlgpu_grid_desc *gd,
                                void *stream) {
   Geom g;
-  ARL_TRY(make_geom(gd, cd, precision, &g));
+  ARL_TRY(make_geom(gd, cd, precision, nvis, &g));
   if (nvis < 0) return fail(ARLGPU_ERR_INVALID, "nvis < 0");
   if (nvis == 0) return ARLGPU_OK;
   if (!uvw || !frequency || !weight || !wgrid) return fail(ARLGPU_ERR_INVALID, "null array argument");

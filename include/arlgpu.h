@@ -94,9 +94,11 @@ unsigned long long arlgpu_kernel_launches(void);
  *                   2 = as 0, specialised on npol with 32-bit incremental offsets,
  *                   3 = as 2 without the compensation (measurement only: FP32C
  *                       promises compensated sums, so the autotuner never picks it),
- *                   4 = FP32C tiles summed in two-limb 32-bit fixed point: the rounded
- *                       contributions and their rounding residuals (default; needs cf
- *                       tap_absmax; FP64 and an unknown bound use 2),
+ *                   4 = the default: one warp per tile with a subgrid of its own where that is
+ *                       the faster (one support: FP32C with one polarisation, up to 8 taps
+ *                       and from 2 Mi rows; FP64 with one or two, up to 10 taps), else FP32C
+ *                       tiles summed in two-limb 32-bit fixed point: the rounded
+ *                       contributions and their rounding residuals (needs cf tap_absmax; FP64 and an unknown bound use 2),
  *                   5 = as 4 without the residual plane (measurement only)
  *   "degrid_kernel" 0 = one warp per row, 1 = 32-row batches per warp,
  *                   2 = one warp per row, specialised on npol, groups of four steps,
@@ -105,7 +107,8 @@ unsigned long long arlgpu_kernel_launches(void);
  *                   4 = as 3 with the grid tile and each row's kernel taps brought into shared
  *                       memory by TMA tensor copies (FP32C, one polarisation, support <= 32,
  *                       subgrid 48, 16-byte aligned tables, even nx; otherwise 3)
- *   "subgrid"       subgrid edge in cells (16..128), 0 = automatic (48, or 32 when 4 pols)
+ *   "subgrid"       subgrid edge in cells (16..128), 0 = automatic (48; 32 with more pols than one or with
+ *                   one pol, one support up to 8, 2 Mi rows and no more bins than rows)
  *   "chunk"         sorted rows per gridder / degridder CTA (32..2^20, default 512)
  *   "persistent"    1 = the lean and fixed-point kernels run as one grid of resident CTAs,
  *                   each looping over every gridDim-th chunk; 2 = the same resident grid fed by
