@@ -1713,9 +1713,10 @@ __device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsign
 //   FP32C, 1 pol, S = 10 (four taps a lane)    1413 -> 1514: not taken
 //   FP32C, 2 or 4 pols, S = 8                  555 -> 694, 817 -> 1881: not taken
 //   FP32C, 1 pol, 25 M rows, 32 slices         6229 -> 3588
-//   FP64, 1 pol, 1.95 M rows, S = 8 / 10       1921 -> 958, 3335 -> 1810
-//   FP64, 2 pols, 1.95 M rows, S = 8 / 10      3735 -> 1886, 6570 -> 3549
+//   FP64, 1 pol, 1.95 M rows, S = 8 / 10       1898 -> 1050, 3310 -> 1797
+//   FP64, 2 pols, 1.95 M rows, S = 8 / 10      3684 -> 1498, 6517 -> 2721
 //   FP64, 1 pol, S = 12                        1136 -> 1236: not taken
+// (FP64 with real taps; whole products, four FMAs a tap, take 1.5 times as long.)
 template <typename R> struct OwnCell;
 __device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ bool finite_bits(float x) { return (__float_as_int(x) & 0x7f800000) != 0x7f800000; }
@@ -1898,10 +1899,16 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
 #pragma unroll
               for (int u = 0; u < STEPS; ++u)
                 if (cofs[u] >= 0) o[u] = c[cofs[u]];
+              // a branch: as a select both sides used the FP64 unit (invert_2d of 1 M rows, 2 pols: 1400 -> 890 us)
+              if (rl) {
 #pragma unroll
-              for (int u = 0; u < STEPS; ++u)
-                if (cofs[u] >= 0)
-                  c[cofs[u]] = rl ? OwnCell<R>::add_real(o[u], tp[r][u], vw) : OwnCell<R>::add(o[u], tp[r][u], vw);
+                for (int u = 0; u < STEPS; ++u)
+                  if (cofs[u] >= 0) c[cofs[u]] = OwnCell<R>::add_real(o[u], tp[r][u], vw);
+              } else {
+#pragma unroll
+                for (int u = 0; u < STEPS; ++u)
+                  if (cofs[u] >= 0) c[cofs[u]] = OwnCell<R>::add(o[u], tp[r][u], vw);
+              }
             }
           }
         };
