@@ -2146,10 +2146,34 @@ k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restric
               tp[u] = on[u] ? kl[p * ps + t + LP * u + j[u] * dk] : czero<CT>();
               gv[u] = on[u] ? gl[p * pstride + t + LP * u + j[u] * dg] : czero<CT>();
             }
+            if constexpr (sizeof(R) == 8) {
+              // The FP64 unit bounds this: four FMAs a tap, two where this lane's taps are
+              // real (a PSWF's) and no grid value makes a NaN of a zero tap.  3 M rows, S = 8:
+              // 2393 -> 1342 us with one polarisation, 4769 -> 2692 with two.
+              bool real = true;
   #pragma unroll
-            for (int u = 0; u < K; ++u) {
-              ax[p] += gv[u].x * tp[u].x - gv[u].y * tp[u].y;
-              ay[p] += gv[u].x * tp[u].y + gv[u].y * tp[u].x;
+              for (int u = 0; u < K; ++u)
+                real = real && (__double_as_longlong((double)tp[u].y) << 1) == 0 && finite_bits((double)gv[u].x) &&
+                       finite_bits((double)gv[u].y);
+              if (real) {
+  #pragma unroll
+                for (int u = 0; u < K; ++u) {
+                  ax[p] = fma(gv[u].x, tp[u].x, ax[p]);
+                  ay[p] = fma(gv[u].y, tp[u].x, ay[p]);
+                }
+              } else {
+  #pragma unroll
+                for (int u = 0; u < K; ++u) {
+                  ax[p] = fma(gv[u].x, tp[u].x, fma(-gv[u].y, tp[u].y, ax[p]));
+                  ay[p] = fma(gv[u].x, tp[u].y, fma(gv[u].y, tp[u].x, ay[p]));
+                }
+              }
+            } else {
+  #pragma unroll
+              for (int u = 0; u < K; ++u) {
+                ax[p] += gv[u].x * tp[u].x - gv[u].y * tp[u].y;
+                ay[p] += gv[u].x * tp[u].y + gv[u].y * tp[u].x;
+              }
             }
           }
         };

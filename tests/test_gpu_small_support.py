@@ -121,3 +121,20 @@ def test_non_finite_visibilities_reach_their_cells(arl, oracle, precision, rows)
     got = gd.data[0, 0, 0]
     assert not numpy.isfinite(got.real[hit]).any() and not numpy.isfinite(got.imag[hit]).any()
     assert numpy.isfinite(got[~hit]).all()
+
+
+@pytest.mark.parametrize('rows', [1, 200])
+def test_degrid_of_non_finite_cells(arl, oracle, rows):
+    """FP64, real taps: an infinite cell makes its rows non-finite in both parts, as the
+    whole complex product does, and no others."""
+    im, cf, uvw, f, v, w, maps, shape, frame = _case(arl, oracle, rows, 8, 4, 64, 1, 1, False, True, 6)
+    vis = arl.Visibility(uvw=uvw, frequency=f, vis=v, weight=w, imaging_weight=w, polarisation_frame=frame)
+    gd = arl.create_griddata_from_image(im)
+    pu, pv = maps[0].astype(int), maps[2].astype(int)
+    x, y = pu[0] - 1, pv[0] + 2
+    gd.data[...] = 1 + 1j
+    gd.data[0, 0, 0, y, x] = complex(numpy.inf, 1.0)
+    out = arl.degrid_visibility_from_griddata(vis, gd, cf, precision='fp64').vis[:, 0]
+    hit = (x >= pu - 4) & (x < pu + 4) & (y >= pv - 4) & (y < pv + 4)
+    assert hit[0] and not numpy.isfinite(out.real[hit]).any() and not numpy.isfinite(out.imag[hit]).any()
+    assert numpy.isfinite(out[~hit]).all()
