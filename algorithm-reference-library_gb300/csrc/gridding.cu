@@ -1977,8 +1977,12 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
 // (sum re t.re, sum re t.im) and (sum im t.re, sum im t.im), instead of four.
 // STASH (with a chunk of at most kStashRows rows and a cf table of fewer than
 // 2^31 taps): the footprint pass leaves each row's set-up in shared memory.
+//
+// Three CTAs an SM with four polarisations and 8 or 16 lanes a row: their subgrids
+// take 64 KiB each, and with the 102 registers a thread that the compiler otherwise
+// gives itself two fit (12.6 M rows x 4: 3736 against 4096 us).
 template <typename R, int NPOL, int NW, bool DUP = false, int LPR = 0, int SGC = 0, bool STASH = false>
-__global__ void __launch_bounds__(NW * 32)
+__global__ void __launch_bounds__(NW * 32, NPOL == 4 && SGC == 32 && (LPR == 8 || LPR == 16) ? 3 : 0)
 k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__ sidx,
               const uint32_t *__restrict__ off, uint32_t chunk, int64_t nvis,
               const typename Cplx<R>::T *__restrict__ cf, const typename Cplx<R>::T *__restrict__ grid,
