@@ -3280,6 +3280,7 @@ static int launch_degrid_tma(const Geom &g, const PlanBufs &b, int64_t nvis, con
                                           static_cast<float2 *>(vis_out), queue, b.queue + 2);
   ARL_LAUNCH_CHECK();
   count_launch(1);
+  *launched = true;
   return ARLGPU_OK;
 }
 
