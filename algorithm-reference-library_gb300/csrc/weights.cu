@@ -126,9 +126,12 @@ k_grid_weight(const double *__restrict__ uvw, const double *__restrict__ freq, c
 }
 
 // w / sum.  An FP64 division takes the FP64 unit 9 operations' time; a
-// FP32 weight's quotient comes from a double-single one instead (48 bits before
+// FP32 weight's quotient comes from a double-single one instead (46 bits before
 // its one rounding to FP32) when the sum's magnitude leaves room for the
-// low parts.
+// low parts.  Where it lies within 1e-4 of half an ulp of a rounding boundary,
+// so that those bits might not decide it (Ziv's test: the sum with the low part
+// enlarged rounds otherwise), the division does: the result is always the FP64
+// quotient's.
 __device__ __forceinline__ double divide(double w, double sum) { return w / sum; }
 __device__ __forceinline__ float divide(float w, double sum) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(sum);
@@ -141,6 +144,7 @@ __device__ __forceinline__ float divide(float w, double sum) {
   if (w == 0.f) return __fdiv_rn(w, hi);  // a flagged row's zero keeps its sign
   const float unit = __uint_as_float((unsigned)((b >> 63) << 31) | (unsigned)(e - 1023 + 127 - 52) << 23);
   const dsf q = ds_div({w, 0.f}, quick_two_sum(hi, (float)((unsigned)b & 0x1fffffffu) * unit));
+  if (__fadd_rn(q.hi, __fmul_rn(q.lo, 1.0001f)) != q.hi) return (float)((double)w / sum);
   return q.hi;
 }
 
