@@ -347,7 +347,7 @@ k_dsfft_rows(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t
   // Rows (or the half's sums) that are all zero, common in w-stack slices, transform to zero.
   bool nz = false;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) nz = nz || (x[j].h & 0x7fffffff7fffffffull) != 0;
+  for (int j = 0; j < 16; ++j) nz = nz || ((x[j].h | x[j].l) & 0x7fffffff7fffffffull) != 0;  // w-planes may cancel in h
   if (!__syncthreads_or(nz)) {
     for (int t = threadIdx.x; t < kRowPts; t += kRowT) {
       const int64_t R = row0 + (t >> LX);
