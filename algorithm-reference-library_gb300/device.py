@@ -227,11 +227,16 @@ def fft_image_to_grid(image_t, gcf_t, gd, precision, out=None, stream=None):
     return out
 
 
-def to_device(a, dtype, device, non_blocking=True):
+def to_device(a, dtype, device, non_blocking=False):
     """Host NumPy array -> device tensor.  Straight from the array's own pages: a
     pinned copy first costs a pass over the data (0.35 ms for 7 MB) and the driver
-    stages pageable memory at the link's rate."""
-    return torch.from_numpy(numpy.ascontiguousarray(a)).to(dtype).to(device, non_blocking=non_blocking)
+    stages pageable memory at the link's rate.  The copy has left the host's memory
+    on return (a host whose pages the GPU can read need not stage them, and ``a``
+    may be a temporary); with ``non_blocking`` it is queued from a pinned snapshot."""
+    t = torch.from_numpy(numpy.ascontiguousarray(a)).to(dtype)
+    if non_blocking and device.type == 'cuda':
+        return t.pin_memory().to(device, non_blocking=True)
+    return t.to(device)
 
 
 _UNPACK_ROWS = 1 << 22
