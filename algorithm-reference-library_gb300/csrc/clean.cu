@@ -271,6 +271,7 @@ k_hogbom(HogArgs a) {
       }
       bv = __shfl_sync(0xffffffffu, bv, leader);
       w1 = __shfl_sync(0xffffffffu, w1, leader);
+      __syncwarp();  // orders the leader's lookup value and its fence before the other lanes' slots
       if (lane < kHogCopies) hog_put(slot + 2 * ((size_t)lane * G + cta), bv | mark, w1);
       // Everybody's best pixel, kHogPoll slots a lane, all loads of a round in flight together; the key (segment,
       // pixel in it) orders pixels as the image does.
