@@ -407,13 +407,10 @@ def deconvolve_cube(dirty, psf, prefix='', **kwargs):
 def _deconvolve_planes(dirty, psf, algorithm, prefix, kwargs):
     """One 'hogbom' or 'msclean' per (channel, polarisation), each plane on the device
     from its own array or tensor; the results come back into the host cubes once."""
-    device = dv.require_cuda()
     shape = tuple(dirty.data.shape)
     mask = get_parameter(kwargs, 'mask', None)
     edge = get_parameter(kwargs, 'window_edge', 16)
     window = clean_window(shape[2:], get_parameter(kwargs, 'window_shape', None), edge)
-    if window is not None:
-        window = _plane(window, device)
     masks = mask.data if isinstance(mask, Image) else None
     crop_psf_to_support(psf, get_parameter(kwargs, 'psf_support', max(shape[2] // 2, shape[3] // 2)))
     gain = get_parameter(kwargs, 'gain', 0.7)
@@ -425,9 +422,16 @@ def _deconvolve_planes(dirty, psf, algorithm, prefix, kwargs):
     scales = get_parameter(kwargs, 'scales', [0, 3, 10, 30])
     fracthresh = get_parameter(kwargs, 'fractional_threshold', 0.01 if algorithm == 'msclean' else 0.1)
     assert 0.0 < fracthresh < 1.0
+    for im in (dirty, psf):
+        if isinstance(im.data, torch.Tensor) and im.data.requires_grad:
+            raise RuntimeError('deconvolve_cube %s: CLEAN has no gradient; detach the image first' % prefix)
     comp = numpy.zeros(shape)
     resid = numpy.zeros(shape)
-    for ch in range(shape[0]):
+    blank = isinstance(psf.data, numpy.ndarray) and not psf.data.any()
+    device = None if blank else dv.require_cuda()
+    if window is not None and not blank:
+        window = _plane(window, device)
+    for ch in range(0 if blank else shape[0]):
         for pol in range(shape[1]):
             p = _plane(psf.data[ch, pol], device)
             if not float(p.max().item()):
