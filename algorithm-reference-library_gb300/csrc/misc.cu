@@ -62,7 +62,7 @@ __global__ void k_gains(CT *vis, int64_t nvis, int npol, const int32_t *a1, cons
 //   d/d conj(g[a2]) = -g1 sum Q            (over rows and pols)
 //   d/d conj(g[a1]) = -g2 conj(sum Q)
 // Bound by the FP64 unit (2 operations a clock and SM), so the row's work is
-// kept to 14 multiply-adds: a thread takes kChiRows consecutive rows, forms the
+// kept to 14 multiply-adds: a thread takes ROWS consecutive rows, forms the
 // gain product once per run of one baseline (the channels of a time, in the
 // usual row order) and sums Q over the run, and the two gain derivatives follow
 // from the run's sum.  The a1 derivative is summed while a1 stays and then, when
@@ -70,12 +70,14 @@ __global__ void k_gains(CT *vis, int64_t nvis, int npol, const int32_t *a1, cons
 // an FP64 addition to shared memory is a compare-and-swap loop that 32 lanes on
 // one word would run 32 times over.
 // 15.6 M rows, 128 antennas, 8 channels: 3882 -> 790 us.
-constexpr int kChiRows = 8;
-
+// ROWS is 8 where that gives more than every second SM a block, 4 down to 64 Ki rows,
+// and 1 below, where few rows a thread keep its chain of waits short.  8 / 4 / 1 rows, us, 64
+// antennas: 3,000 rows of one channel 33 / 21 / 16 (in random order 38 / 23 / 12),
+// 100,000 rows 34 / 23 / 32 (39 / 25 / 27), 300,000 rows 35 / 40 / 66 (40 / 42 / 42).
 template <typename CT> struct ChiPair { using T = double4; };
 template <> struct ChiPair<float2> { using T = float4; };
 
-template <typename CT, int NPOL>
+template <typename CT, int NPOL, int ROWS>
 __global__ void __launch_bounds__(256)
 k_gain_chi2(const CT *__restrict__ vobs, const CT *__restrict__ m, const double *__restrict__ wt, int64_t nvis,
             int npol_arg, const int32_t *__restrict__ a1, const int32_t *__restrict__ a2,
@@ -85,12 +87,12 @@ k_gain_chi2(const CT *__restrict__ vobs, const CT *__restrict__ m, const double 
   for (int i = threadIdx.x; i < 2 * nant; i += blockDim.x) sg[i] = 0.0;
   __syncthreads();
   const int npol = NPOL ? NPOL : npol_arg, lane = threadIdx.x & 31;
-  const int64_t nrun = (nvis + kChiRows - 1) / kChiRows;
+  const int64_t nrun = (nvis + ROWS - 1) / ROWS;
   // whole warps loop together: the flush at the end of a run is a warp's
   const int64_t first = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31;
   double local = 0.0;
   for (int64_t w0 = first; w0 < nrun; w0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t rb = (w0 + lane) * kChiRows, re = min(rb + kChiRows, nvis);
+    const int64_t rb = (w0 + lane) * ROWS, re = min(rb + ROWS, nvis);
     int c1 = -1, c2 = -1;
     double2 g1{}, g2{};
     double gr = 0.0, gi = 0.0, qx = 0.0, qy = 0.0, dx = 0.0, dy = 0.0;
@@ -137,10 +139,10 @@ k_gain_chi2(const CT *__restrict__ vobs, const CT *__restrict__ m, const double 
       gr = g2.x * g1.x + g2.y * g1.y;  // g2 conj(g1)
       gi = g2.y * g1.x - g2.x * g1.y;
     };
-    if (NPOL == 1 && pairs && rb + kChiRows <= nvis) {
+    if (NPOL == 1 && ROWS % 2 == 0 && pairs && rb + ROWS <= nvis) {
       using P = typename ChiPair<CT>::T;
 #pragma unroll
-      for (int j = 0; j < kChiRows; j += 2) {
+      for (int j = 0; j < ROWS; j += 2) {
         const int2 i1 = *reinterpret_cast<const int2 *>(a1 + rb + j), i2 = *reinterpret_cast<const int2 *>(a2 + rb + j);
         const P vo = *reinterpret_cast<const P *>(vobs + rb + j), mo = *reinterpret_cast<const P *>(m + rb + j);
         CT g0{}, g1o{};
@@ -190,22 +192,31 @@ k_gain_chi2(const CT *__restrict__ vobs, const CT *__restrict__ m, const double 
       }
 }
 
+template <typename CT, int ROWS>
+static void launch_gain_chi2_rows(const CT *vo, const CT *mo, const double *wt, int64_t nvis, int npol,
+                                  const int32_t *a1, const int32_t *a2, const double2 *g, int nant, double *chi2,
+                                  CT *gm, double2 *grad_g, int pairs, cudaStream_t st) {
+  const int64_t want = ((nvis + ROWS - 1) / ROWS + 255) / 256;
+  const int blocks = (int)(want < 152 * 4 ? want : 152 * 4);
+  const size_t smem = 2 * sizeof(double) * nant;
+  if (npol == 1)
+    k_gain_chi2<CT, 1, ROWS><<<blocks, 256, smem, st>>>(vo, mo, wt, nvis, npol, a1, a2, g, nant, chi2, gm, grad_g, pairs);
+  else
+    k_gain_chi2<CT, 0, ROWS><<<blocks, 256, smem, st>>>(vo, mo, wt, nvis, npol, a1, a2, g, nant, chi2, gm, grad_g, pairs);
+}
+
 template <typename CT>
 static void launch_gain_chi2(const void *vobs, const void *model, const double *wt, int64_t nvis, int npol,
                              const int32_t *a1, const int32_t *a2, const double2 *g, int nant, double *chi2,
                              void *grad_m, double2 *grad_g, cudaStream_t st) {
-  const int64_t want = ((nvis + kChiRows - 1) / kChiRows + 255) / 256;
-  const int blocks = (int)(want < 152 * 4 ? want : 152 * 4);
-  const size_t smem = 2 * sizeof(double) * nant;
-  // two rows in one 16-byte access: the arrays' first elements decide, rows are taken 8 at a time
+  // two rows in one 16-byte access: the arrays' first elements decide, rows are taken an even number at a time
   auto at = [](const void *p, uintptr_t n) { return ((uintptr_t)p & (n - 1)) == 0; };
   const int pairs = sizeof(CT) == 8 && at(vobs, 16) && at(model, 16) && at(grad_m, 16) && at(a1, 8) && at(a2, 8);
   const CT *vo = static_cast<const CT *>(vobs), *mo = static_cast<const CT *>(model);
   CT *gm = static_cast<CT *>(grad_m);
-  if (npol == 1)
-    k_gain_chi2<CT, 1><<<blocks, 256, smem, st>>>(vo, mo, wt, nvis, npol, a1, a2, g, nant, chi2, gm, grad_g, pairs);
-  else
-    k_gain_chi2<CT, 0><<<blocks, 256, smem, st>>>(vo, mo, wt, nvis, npol, a1, a2, g, nant, chi2, gm, grad_g, pairs);
+  auto launch = nvis < 65536 ? launch_gain_chi2_rows<CT, 1>
+                             : nvis <= 4 * 152 * 256 ? launch_gain_chi2_rows<CT, 4> : launch_gain_chi2_rows<CT, 8>;
+  launch(vo, mo, wt, nvis, npol, a1, a2, g, nant, chi2, gm, grad_g, pairs, st);
 }
 
 // apply_gaintable with scalar gains on a BlockVisibility (one polarisation):
