@@ -452,7 +452,11 @@ __device__ __forceinline__ SegInfo seg_at(uint32_t pos, uint32_t c1, const RowMa
   RowMap m = smap[pos];
   s.ch = m.cz & 0xffff;
   s.zg = m.cz >> 16;
-  uint32_t key = bin_of(s.ch, s.zg, m.pu, m.pv, g);
+  // bin_of by the quotients that u0 and v0 need.  The form matters to the packed
+  // degridder's registers: this one gives it 80 with four polarisations (three CTAs an
+  // SM) and 32 with one and large supports, bin_of's high words or the quotients in
+  // variables 102 and 49 (71.9 M rows x 4 pols: 15.5 against 17.8 ms).
+  const uint32_t key = (((uint32_t)s.ch * g.nw + s.zg) * g.ntv + m.pv / g.T) * g.ntu + m.pu / g.T;
   s.end = min(off[key + 1], c1);
   s.u0 = (m.pu / g.T) * g.T - (g.S >> 1);
   s.v0 = (m.pv / g.T) * g.T - (g.S >> 1);
@@ -1977,12 +1981,8 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
 // (sum re t.re, sum re t.im) and (sum im t.re, sum im t.im), instead of four.
 // STASH (with a chunk of at most kStashRows rows and a cf table of fewer than
 // 2^31 taps): the footprint pass leaves each row's set-up in shared memory.
-//
-// Three CTAs an SM with four polarisations and 8 or 16 lanes a row: their subgrids
-// take 64 KiB each, and with the 102 registers a thread that the compiler otherwise
-// gives itself two fit (12.6 M rows x 4: 3736 against 4096 us).
 template <typename R, int NPOL, int NW, bool DUP = false, int LPR = 0, int SGC = 0, bool STASH = false>
-__global__ void __launch_bounds__(NW * 32, NPOL == 4 && SGC == 32 && (LPR == 8 || LPR == 16) ? 3 : 0)
+__global__ void __launch_bounds__(NW * 32)
 k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__ sidx,
               const uint32_t *__restrict__ off, uint32_t chunk, int64_t nvis,
               const typename Cplx<R>::T *__restrict__ cf, const typename Cplx<R>::T *__restrict__ grid,
