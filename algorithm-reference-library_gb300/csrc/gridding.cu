@@ -64,17 +64,19 @@ static std::atomic<int> g_tune_stash{1};          // packed degridder, one polar
 void count_launch(unsigned n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 bool tune_dsfft() { return g_tune_dsfft.load() != 0; }
 
-// K1: mapping + histogram + each row's rank within its bin.  A thread takes ROWS
-// (4, or 1 where that would leave SMs idle) rows a block width apart, all loads
-// first.  The atomic's returned count gives the rank, so the scatter needs no
-// atomic of its own, and no second clearing of the histogram.  The rows of a warp in
-// one bin share an atomic, wherever they lie in it: rows in no order that fall into
-// few bins otherwise queue at a few addresses (2.2 M rows over 30 or 200 pixels, runs of
-// neighbouring rows found by comparing with the row before: 745 -> 115 and 376 -> 284
-// us; 121 k rows of a 512^2 image 27.3 -> 17.7 us; rows in baseline order unchanged).
-// 4.3 M rows of the w-projection plan: k_map 117 -> 97 us (350 instructions a row
-// and two memory latencies), k_scatter 125 -> 96 us, k_scan 13.7 -> 6.5 us, the second
-// clearing gone.
+// K1: mapping + histogram + each row's rank within its bin.  The atomic's returned
+// count gives the rank, so the scatter needs no atomic of its own, and no second
+// clearing of the histogram.  The rows of a warp in one bin share an atomic, wherever
+// they lie in it: rows in no order that fall into few bins otherwise queue at a few
+// addresses (2.2 M rows over 30 or 200 pixels, runs of neighbouring rows found by
+// comparing with the row before: 745 -> 115 and 376 -> 284 us; 121 k rows of a 512^2
+// image 27.3 -> 17.7 us; rows in baseline order unchanged).  A thread a row, here and
+// in k_scatter: with four rows a thread k_map takes 64 registers instead of 42, and its
+// fewer, longer blocks hold up another stream's gridder (4.3 M rows of the
+// w-projection plan, k_map / k_scatter: 112 / 80 us against 116 / 97, and 3.296
+// against 3.318 ms a step for two streams of plan, grid and degrid with copies).  A
+// grid of resident blocks that loop over rows mixes the rows of a bin, which costs the
+// gridder 1 % (1387 against 1371 us).
 __device__ __forceinline__ RowMap row_map(const Mapped &m) {
   RowMap rm;
   rm.pu = m.ok ? m.pu : -1;  // a rejected row
@@ -84,64 +86,25 @@ __device__ __forceinline__ RowMap row_map(const Mapped &m) {
   return rm;
 }
 
-template <int ROWS>
 __global__ void __launch_bounds__(256)
 k_map(const double *__restrict__ uvw, const double *__restrict__ freq, int64_t nvis, Geom g,
       uint32_t *__restrict__ ranks, RowMap *__restrict__ maps, uint32_t *__restrict__ hist) {
   const int lane = threadIdx.x & 31;
-  const int64_t r0 = (int64_t)blockIdx.x * (256 * ROWS) + threadIdx.x;
-  RowMap rm[ROWS];
-  uint32_t undecided = 0;
-  {
-    double u[ROWS], v[ROWS], w[ROWS], f[ROWS];
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      const int64_t r = min(r0 + 256 * j, nvis - 1);
-      u[j] = uvw[3 * r];
-      v[j] = uvw[3 * r + 1];
-      w[j] = uvw[3 * r + 2];
-      f[j] = freq[r];
-    }
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      Mapped m{};
-      if (!map_row_fixed(u[j], v[j], w[j], f[j], g, &m)) undecided |= 1u << j;
-      rm[j] = row_map(m);
-    }
-  }
-  // Rows near a boundary, a few in a million: their FP64 sequences are kept in one
-  // place, after the coordinates' registers are free.
-#pragma unroll 1
-  while (undecided) {
-    const int j = __ffs(undecided) - 1;
-    undecided &= undecided - 1;
-    const int64_t r = min(r0 + 256 * j, nvis - 1);
-    const RowMap x = row_map(map_row_exact(uvw[3 * r], uvw[3 * r + 1], uvw[3 * r + 2], freq[r], g));
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k)
-      if (k == j) rm[k] = x;
-  }
+  const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x, at = min(r, nvis - 1);
+  Mapped m{};
+  if (!map_row_fixed(uvw[3 * at], uvw[3 * at + 1], uvw[3 * at + 2], freq[at], g, &m))
+    m = map_row_exact(uvw[3 * at], uvw[3 * at + 1], uvw[3 * at + 2], freq[at], g);
   __syncwarp();
-  uint32_t start[ROWS], lead[ROWS], below[ROWS];
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const int64_t r = r0 + 256 * j;
-    const uint32_t key = r >= nvis ? 0xffffffffu
-                                   : (rm[j].pu < 0 ? g.nbins
-                                                   : bin_of(rm[j].cz & 0xffff, rm[j].cz >> 16, rm[j].pu, rm[j].pv, g));
-    if (r < nvis) st_map16(maps + r, rm[j]);
-    const uint32_t peers = __match_any_sync(0xffffffffu, key);
-    lead[j] = __ffs(peers) - 1;
-    below[j] = __popc(peers & ((1u << lane) - 1));
-    start[j] = 0;
-    if (lead[j] == (uint32_t)lane && key != 0xffffffffu) start[j] = atomicAdd(&hist[key], (uint32_t)__popc(peers));
-  }
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const int64_t r = r0 + 256 * j;
-    const uint32_t s = __shfl_sync(0xffffffffu, start[j], lead[j]);
-    if (r < nvis) ranks[r] = s + below[j];
-  }
+  const RowMap rm = row_map(m);
+  const uint32_t key = r >= nvis ? 0xffffffffu
+                                 : (rm.pu < 0 ? g.nbins : bin_of(rm.cz & 0xffff, rm.cz >> 16, rm.pu, rm.pv, g));
+  if (r < nvis) st_map16(maps + r, rm);
+  const uint32_t peers = __match_any_sync(0xffffffffu, key);
+  const int lead = __ffs(peers) - 1;
+  uint32_t start = 0;
+  if (lane == lead && key != 0xffffffffu) start = atomicAdd(&hist[key], (uint32_t)__popc(peers));
+  start = __shfl_sync(0xffffffffu, start, lead);
+  if (r < nvis) ranks[r] = start + __popc(peers & ((1u << lane) - 1));
 }
 
 // Mapping export for arlgpu_convolution_mapping: the same indices the plan
@@ -298,31 +261,17 @@ __global__ void k_scan_add(uint32_t *__restrict__ off, uint32_t n, const uint32_
   if (i < n) off[i] += tile_sum[i / kScanTile];
 }
 
-// K2b: rows into bin order by bin offset and rank; ROWS rows a thread, as k_map.
-template <int ROWS>
+// K2b: rows into bin order by bin offset and rank.
 __global__ void __launch_bounds__(256)
 k_scatter(const uint32_t *__restrict__ ranks, const RowMap *__restrict__ maps, int64_t nvis, Geom g,
           const uint32_t *__restrict__ off, uint32_t *__restrict__ sidx, RowMap *__restrict__ smap) {
-  const int64_t r0 = (int64_t)blockIdx.x * (256 * ROWS) + threadIdx.x;
-  RowMap m[ROWS];
-  uint32_t pos[ROWS];
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const int64_t r = min(r0 + 256 * j, nvis - 1);
-    m[j] = ld_map16(maps + r);
-    pos[j] = ranks[r];
-  }
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j)
-    pos[j] += off[m[j].pu < 0 ? g.nbins : bin_of(m[j].cz & 0xffff, m[j].cz >> 16, m[j].pu, m[j].pv, g)];
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    const int64_t r = r0 + 256 * j;
-    if (r < nvis) {
-      sidx[pos[j]] = (uint32_t)r;  // the rejected rows come last: the degridder zeroes their output
-      st_map16(smap + pos[j], m[j]);
-    }
-  }
+  const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (r >= nvis) return;
+  const RowMap m = ld_map16(maps + r);
+  const uint32_t key = m.pu < 0 ? g.nbins : bin_of(m.cz & 0xffff, m.cz >> 16, m.pu, m.pv, g);
+  const uint32_t pos = off[key] + ranks[r];
+  sidx[pos] = (uint32_t)r;  // the rejected rows come last: the degridder zeroes their output
+  st_map16(smap + pos, m);
 }
 
 // Mean w of the rows of each grid w-plane (over all channels), from a built
@@ -2937,15 +2886,10 @@ static int num_sms() {
 int plan_build(const double *uvw, const double *freq, int64_t nvis, const Geom &g, const PlanBufs &b,
                int64_t *n_bad_dev, cudaStream_t st) {
   const uint32_t nh = g.nbins + 1;
-  // four rows a thread once that still gives every SM two blocks
-  const bool four = nvis >= (int64_t)2 * 1024 * num_sms();
-  const unsigned plan_blocks = (unsigned)((nvis + (four ? 1023 : 255)) / (four ? 1024 : 256));
+  const unsigned plan_blocks = (unsigned)((nvis + 255) / 256);
   ARL_CUDA(cudaMemsetAsync(b.hist, 0, (size_t)nh * 4, st));
   if (nvis > 0) {
-    if (four)
-      k_map<4><<<plan_blocks, 256, 0, st>>>(uvw, freq, nvis, g, b.keys, b.maps, b.hist);
-    else
-      k_map<1><<<plan_blocks, 256, 0, st>>>(uvw, freq, nvis, g, b.keys, b.maps, b.hist);
+    k_map<<<plan_blocks, 256, 0, st>>>(uvw, freq, nvis, g, b.keys, b.maps, b.hist);
     ARL_LAUNCH_CHECK();
     count_launch(1);
   }
@@ -2969,10 +2913,7 @@ int plan_build(const double *uvw, const double *freq, int64_t nvis, const Geom &
     count_launch(3);
   }
   if (nvis > 0) {
-    if (four)
-      k_scatter<4><<<plan_blocks, 256, 0, st>>>(b.keys, b.maps, nvis, g, b.offsets, b.sidx, b.smap);
-    else
-      k_scatter<1><<<plan_blocks, 256, 0, st>>>(b.keys, b.maps, nvis, g, b.offsets, b.sidx, b.smap);
+    k_scatter<<<plan_blocks, 256, 0, st>>>(b.keys, b.maps, nvis, g, b.offsets, b.sidx, b.smap);
     ARL_LAUNCH_CHECK();
     count_launch(1);
   }
