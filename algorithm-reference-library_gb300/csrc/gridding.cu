@@ -2239,6 +2239,91 @@ k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restric
   }
 }
 
+// K4 (rows; plans of small subgrids, one polarisation and one support up to 8).
+// A plan of 32-cell subgrids has up to 2.8 times the bins of one of 48, and what the
+// packed degridder spends its time on where few rows share a bin is the bins: set-up,
+// footprint pass, staging and two barriers each.  Here a warp takes 32 sorted rows, one
+// per lane for their set-up and eight lanes a row for the taps; the cells come from the
+// grid through L1, where the rows of a bin find each other's (eight lanes read 64 bytes of
+// a window's row as they read 128 from a staged one).  No barriers, no shared memory, and all
+// of a row's loads in flight.  us, S = 8, FP32C, packed with 48 cells / with 32 / this:
+//   3 M rows, 4096^2, 20 slices      1521 / 2662 /  479
+//   12 M rows, 4096^2, 20 slices     3320 / 4505 / 1219
+//   2.2 M rows over 1800^2 pixels     253 /  250 /  163
+//   8.8 M rows over 1800^2 pixels     905 /  840 /  615
+// FP64, real taps: 3 M rows 3273 / 4628 / 1373; 12 M rows 10405 / 8862 / 5364.
+template <typename R, int STEPS>
+__global__ void __launch_bounds__(256)
+k_degrid_rows(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__ sidx,
+              const uint32_t *__restrict__ off, int64_t nvis, const typename Cplx<R>::T *__restrict__ cf,
+              const typename Cplx<R>::T *__restrict__ grid, typename Cplx<R>::T *__restrict__ vis_out) {
+  using CT = typename Cplx<R>::T;
+  const int lane = threadIdx.x & 31, hl = lane & 7, S = g.S, n = S * S;
+  const int64_t r0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) & ~(int64_t)31;  // the warp's first row
+  if (r0 >= nvis) return;
+  const int64_t r = r0 + lane, nvalid = off[g.nbins];
+  const uint32_t idx = r < nvis ? sidx[r] : 0;
+  CT out = czero<CT>();  // rows that the plan rejected stay zero
+  if (r0 < nvalid) {
+    int gofs[STEPS];  // this lane's cells in the window; -1: no tap
+#pragma unroll
+    for (int u = 0; u < STEPS; ++u) {
+      const int t = hl + 8 * u;
+      gofs[u] = t < n ? t / S * g.nx + t % S : -1;
+    }
+    const RowMap m = smap[min(r, nvalid - 1)];
+    const int ch = m.cz & 0xffff, zg = m.cz >> 16;
+    const int koff = (int)(ch * g.cf_chan_stride + (int)(m.sub >> 16) * g.cf_z_stride) +
+                     (int)(((m.sub >> 8) & 0xff) * g.O + (m.sub & 0xff)) * n;
+    const int64_t goff = (((int64_t)ch * g.nw + zg) * g.ny + m.pv - (S >> 1)) * g.nx + m.pu - (S >> 1);
+#pragma unroll 2
+    for (int i = 0; i < 8; ++i) {
+      const int src = 4 * i + (lane >> 3);
+      const CT *k = cf + __shfl_sync(0xffffffffu, koff, src) + hl;
+      const CT *c = grid + __shfl_sync(0xffffffffu, goff, src);
+      CT tp[STEPS], gv[STEPS];
+#pragma unroll
+      for (int u = 0; u < STEPS; ++u) {
+        tp[u] = gofs[u] >= 0 ? k[8 * u] : czero<CT>();
+        gv[u] = gofs[u] >= 0 ? c[gofs[u]] : czero<CT>();
+      }
+      R ax = 0, ay = 0;
+      bool real = sizeof(R) == 8;  // FP64, as in k_degrid_lean: two FMAs a tap where this lane's taps are real
+      if constexpr (sizeof(R) == 8) {
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u)
+          real = real && (__double_as_longlong(tp[u].y) << 1) == 0 && finite_bits(gv[u].x) && finite_bits(gv[u].y);
+      }
+      if (real) {
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u) {
+          ax = fma(gv[u].x, tp[u].x, ax);
+          ay = fma(gv[u].y, tp[u].x, ay);
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u) {
+          ax = fma(gv[u].x, tp[u].x, fma(-gv[u].y, tp[u].y, ax));
+          ay = fma(gv[u].x, tp[u].y, fma(gv[u].y, tp[u].x, ay));
+        }
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+      }
+      // to the lane whose row it is
+      ax = __shfl_sync(0xffffffffu, ax, 8 * (lane & 3));
+      ay = __shfl_sync(0xffffffffu, ay, 8 * (lane & 3));
+      if (lane >> 2 == i && r < nvalid) {
+        out.x = ax;
+        out.y = ay;
+      }
+    }
+  }
+  if (r < nvis) vis_out[idx] = out;
+}
+
 // ---------------------------------------------------------------------------
 // K4 (TMA variant, degrid_kernel 4): the packed FP32 degridder with the grid
 // footprint and the kernel taps staged in shared memory by the tensor-memory
@@ -2803,15 +2888,14 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
   }
   SG = fitted(SG);
   // Many rows of one polarisation and one small support: the one-warp gridder wants
-  // many subgrids resident (14 of 32^2 cells an SM against 6 of 48^2).  24 cells, with
-  // 24 resident, grid a little faster, but the degridder, which stages a bin's subgrid,
-  // loses where a bin has few rows.  Nor is it for fewer rows (k_grid_own), or for more
-  // tiles than rows, which would cost the plan more to scan than its rows.  S = 8, us,
-  // subgrid 48 / 32 / 24: grid 2157 / 1717 / 1539 and degrid 1569 / 1491 / 1563 (15.6 M
-  // rows of the gain solve), grid 6229 / 3588 / 3602 (25 M rows, 8192^2, 32 slices),
-  // degrid 1664 / 1655 / 2144 (12.6 M rows, 4096^2, 20 slices), 2.2 M rows spread over
-  // 1800^2 pixels grid 355 / 280 / 279, degrid 257 / 247 / 278.
-  if (!chosen && g->npol == 1 && g->S <= 8 && !g->plane_support && nvis >= kSmallTileRows &&
+  // many subgrids resident (14 of 32^2 cells an SM against 6 of 48^2), and k_degrid_rows
+  // has no use for larger ones.  Not fewer rows (k_grid_own), nor more tiles than
+  // rows, which would cost the plan more to scan than its rows, nor S = 2 (8.8 M rows over
+  // 1800^2 pixels: grid 853 -> 925).  S = 8, us, gridder with subgrid 48 / 32 / 24:
+  // 2157 / 1717 / 1539 (15.6 M rows of the gain solve), 6229 / 3588 / 3602 (25 M rows,
+  // 8192^2, 32 slices), 355 / 280 / 279 (2.2 M rows spread over 1800^2 pixels); 24 cells
+  // would also put more roundings into the grid (k_grid_own's flushes).
+  if (!chosen && g->npol == 1 && g->S >= 4 && g->S <= 8 && !g->plane_support && nvis >= kSmallTileRows &&
       bins(fitted(32)) <= (uint64_t)nvis)
     SG = fitted(32);
   if ((size_t)g->npol * SG * fx_pitch(SG) * cell > 200 * 1024)
@@ -3041,16 +3125,22 @@ static int launch_grid_fx(const Geom &g, const PlanBufs &b, int64_t nvis, const 
   return ARLGPU_OK;
 }
 
+// Plans of small subgrids and many rows (make_geom's choice, or asked for) whose cf table
+// is addressable in 32 bits.
+static bool small_tiles(const Geom &g, int64_t nvis) {
+  return !g.plane_support && g.S >= 4 && g.S <= 8 && g.SG <= 32 && nvis >= kSmallTileRows && cf_elems(g) < 0x7fffffffll;
+}
+
 // Whether the one-warp gridder takes a call (its comment has both sides measured):
 // rows of one support in a cf table addressable in 32 bits, FP32C with one
-// polarisation, S <= 8, the small subgrid and rows enough that their chunks give
+// polarisation, 4 <= S <= 8, the small subgrid and rows enough that their chunks give
 // every warp some (at 1 M rows 156 -> 123 us with 24 cells, at 0.1 M 53 -> 69),
 // FP64 with one or two, S <= 10 and subgrids of at most 36 KiB: six warps an SM (two
 // polarisations with 72 KiB, a subgrid edge of 48 asked for: 2021 -> 2587 us).
 static bool takes_own(const Geom &g, int64_t nvis, bool fp64) {
-  if (g.plane_support || cf_elems(g) >= 0x7fffffffll) return false;
-  return fp64 ? g.npol <= 2 && g.S <= 10 && g.npol * g.SG * g.SG <= 48 * 48
-              : g.npol == 1 && g.S <= 8 && g.SG <= 32 && nvis >= kSmallTileRows;
+  return fp64 ? !g.plane_support && cf_elems(g) < 0x7fffffffll && g.npol <= 2 && g.S <= 10 &&
+                    g.npol * g.SG * g.SG <= 48 * 48
+              : g.npol == 1 && small_tiles(g, nvis);
 }
 
 template <typename R>
@@ -3234,6 +3324,15 @@ static int launch_degrid(const Geom &g, const PlanBufs &b, int64_t nvis, const v
       ARL_TRY(launch_degrid_tma(g, b, nvis, cf, grid, vis_out, st, &launched));
       if (launched) return ARLGPU_OK;
     }
+  }
+  if (g_tune_degrid_kernel.load() >= 3 && g.npol == 1 && small_tiles(g, nvis)) {
+    using CT = typename Cplx<R>::T;
+    auto rows = g.S <= 4 ? k_degrid_rows<R, 2> : g.S <= 6 ? k_degrid_rows<R, 5> : k_degrid_rows<R, 8>;
+    rows<<<(unsigned)((nvis + 255) / 256), 256, 0, st>>>(g, b.smap, b.sidx, b.offsets, nvis, static_cast<const CT *>(cf),
+                                                         static_cast<const CT *>(grid), static_cast<CT *>(vis_out));
+    ARL_LAUNCH_CHECK();
+    count_launch(1);
+    return ARLGPU_OK;
   }
   size_t smem = (size_t)g.npol * g.SG * g.SG * sizeof(typename Cplx<R>::T);
   auto kern = k_degrid<R, kWarps>;
