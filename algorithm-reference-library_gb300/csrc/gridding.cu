@@ -1734,6 +1734,20 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
     uint32_t pos = c0;
     while (pos < c1) {
       const SegInfo sg = seg_at(pos, c1, smap, off, g);
+      // Rows enough to be worth a look at their maps go row by row to the grid only where their windows lie apart:
+      // else every chunk of a dense bin would, and its additions wait for each other (300,000 rows within two
+      // pixels, S = 4, FP64: 1143 us by seg_at's rule alone, 168 now, 239 in k_grid_lean).
+      bool direct = sg.direct;
+      if (direct && sg.end - pos >= 16) {
+        int bx0 = 0x7fffffff, by0 = 0x7fffffff, bx1 = 0, by1 = 0;
+        for (uint32_t r = pos + lane; r < sg.end; r += 32) {
+          const RowMap q = smap[r];
+          bx0 = min(bx0, q.pu), bx1 = max(bx1, q.pu), by0 = min(by0, q.pv), by1 = max(by1, q.pv);
+        }
+        const int bw = __reduce_max_sync(0xffffffffu, bx1) - __reduce_min_sync(0xffffffffu, bx0) + S;
+        const int bh = __reduce_max_sync(0xffffffffu, by1) - __reduce_min_sync(0xffffffffu, by0) + S;
+        direct = (int)(sg.end - pos) * n < bw * bh;
+      }
       CT *tile = grid + ((int64_t)sg.ch * NPOL * g.nw + sg.zg) * plane_elems;
       double wsum[NPOL];
 #pragma unroll
@@ -1791,7 +1805,7 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
         }
         __syncwarp();
         load_map(b0 + 32 + lane);
-        if (sg.direct) {
+        if (direct) {
           load_val(b0 + 32 + lane);
           for (int i = 0; i < cnt; ++i) {
             const Row rw = s_row[i];
@@ -1888,7 +1902,7 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
         for (int o = 16; o > 0; o >>= 1) wsum[p] += __shfl_xor_sync(0xffffffffu, wsum[p], o);
         if (lane == 0 && wsum[p] != 0.0) atomicAdd(&sumwt[sg.ch * NPOL + p], wsum[p]);
       }
-      if (!sg.direct) {
+      if (!direct) {
         // Flush the footprint and clear it.
         __syncwarp();
         x0 = __reduce_min_sync(0xffffffffu, x0);
