@@ -2116,11 +2116,14 @@ k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restric
               // The FP64 unit bounds this: four FMAs a tap, two where this lane's taps are
               // real (a PSWF's) and no grid value makes a NaN of a zero tap.  3 M rows, S = 8:
               // 2393 -> 1342 us with one polarisation, 4769 -> 2692 with two.
-              bool real = true;
+              bool real = false;
+              if (K > 1) {  // in one step (support 2 has no other) the tests cost more than they save
+                real = true;
   #pragma unroll
-              for (int u = 0; u < K; ++u)
-                real = real && (__double_as_longlong((double)tp[u].y) << 1) == 0 && finite_bits((double)gv[u].x) &&
-                       finite_bits((double)gv[u].y);
+                for (int u = 0; u < K; ++u)
+                  real = real && (__double_as_longlong((double)tp[u].y) << 1) == 0 && finite_bits((double)gv[u].x) &&
+                         finite_bits((double)gv[u].y);
+              }
               if (real) {
   #pragma unroll
                 for (int u = 0; u < K; ++u) {
