@@ -295,54 +295,42 @@ k_dsfft_rows(const float2 *__restrict__ grid, int64_t qstride, int nsum, int64_t
   const int ny = 1 << log2ny, half = SPLIT ? blockIdx.x & 1 : 0;
   const int64_t plane = (int64_t)ny << LROW, nrows = (int64_t)np << log2ny;
   const int64_t row0 = SPLIT ? blockIdx.x >> 1 : (int64_t)blockIdx.x * S;
-  // one FP32 value of row q of this CTA, w-planes summed, signed
-  auto in = [&](int64_t R, int x) -> cds {
-    if (R >= nrows) return {0, 0};
-    const int y = (int)(R & (ny - 1));
-    const float2 *src = grid + (q0 + (R >> log2ny)) * qstride + ((int64_t)y << LROW) + x;
-    float2 g = src[0];
-    cds v{pk(g.x, g.y), 0};
-    for (int z = 1; z < nsum; ++z) {
-      g = src[z * plane];
-      v = c_add(v, cds{pk(g.x, g.y), 0});
-    }
-    const float sg = ((x + y) & 1) ? -1.f : 1.f;
-    return {mul2(v.h, pk(sg, sg)), mul2(v.l, pk(sg, sg))};
-  };
+  // Points [j0, j0 + W) of plane z, signed; SPLIT: with the other half's added or subtracted.  All loads are in
+  // flight before any is used.
   cds x[16];
-  if (nsum == 1) {  // all loads in flight before any is used
-    float2 ga[16], gb[SPLIT ? 16 : 1];
+  auto points = [&](auto j0_c, auto w_c, int z) {
+    constexpr int J0 = decltype(j0_c)::value, W = decltype(w_c)::value;
+    float2 ga[W], gb[SPLIT ? W : 1];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+    for (int i = 0; i < W; ++i) {
+      const int j = J0 + i, item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
       const int64_t R = row0 + q;
-      const float2 *src =
-          grid + (q0 + (R >> log2ny)) * qstride + ((R & (ny - 1)) << LROW) + (j % R0) * M0 + m;
-      ga[j] = R < nrows ? src[0] : make_float2(0.f, 0.f);
-      if (SPLIT) gb[SPLIT ? j : 0] = src[1 << LX];
+      const float2 *src = grid + (q0 + (R >> log2ny)) * qstride + z * plane + ((R & (ny - 1)) << LROW) + (j % R0) * M0 + m;
+      ga[i] = R < nrows ? src[0] : make_float2(0.f, 0.f);
+      if (SPLIT) gb[SPLIT ? i : 0] = src[1 << LX];
     }
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
+    for (int i = 0; i < W; ++i) {
+      const int j = J0 + i, item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
       const float sg = ((m + (int)(row0 + q)) & 1) ? -1.f : 1.f;  // M0, ny and 4096 are even
-      x[j] = {mul2(pk(ga[j].x, ga[j].y), pk(sg, sg)), 0};
+      const cds v{mul2(pk(ga[i].x, ga[i].y), pk(sg, sg)), 0};
+      x[j] = z ? c_add(x[j], v) : v;
       if (SPLIT) {
-        const float2 b = gb[SPLIT ? j : 0];
+        const float2 b = gb[SPLIT ? i : 0];
         const cds y{mul2(pk(b.x, b.y), pk(sg, sg)), 0};
         x[j] = half ? c_sub(x[j], y) : c_add(x[j], y);
       }
     }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int item = threadIdx.x + (j / R0) * kRowT, m = item & (M0 - 1), q = item >> G::LOG2M0;
-      const int n = (j % R0) * M0 + m;
-      x[j] = in(row0 + q, n);
-      if (SPLIT) {
-        const cds y = in(row0 + q, n + (1 << LX));
-        x[j] = half ? c_sub(x[j], y) : c_add(x[j], y);
-      }
-    }
+  };
+  points(std::integral_constant<int, 0>(), std::integral_constant<int, 16>(), 0);
+  // Further w-planes four points at a time (the sums take the other loads' registers).  Point by point, plane after
+  // plane, three planes of 8192^2 took 4.35 ms, now 2.62.
+#pragma unroll 1
+  for (int z = 1; z < nsum; ++z) {
+    points(std::integral_constant<int, 0>(), std::integral_constant<int, 4>(), z);
+    points(std::integral_constant<int, 4>(), std::integral_constant<int, 4>(), z);
+    points(std::integral_constant<int, 8>(), std::integral_constant<int, 4>(), z);
+    points(std::integral_constant<int, 12>(), std::integral_constant<int, 4>(), z);
   }
   // Rows (or the half's sums) that are all zero, common in w-stack slices, transform to zero.
   bool nz = false;
