@@ -133,8 +133,8 @@ __device__ __forceinline__ unsigned long long hog_value(double r, int code, cons
   return a > 0x7ff0000000000000ull ? ~0ull : a;
 }
 
-__device__ __forceinline__ int hog_code(const double *window, long long px) {
-  const unsigned long long w = (unsigned long long)__double_as_longlong(window[px]);
+__device__ __forceinline__ int hog_code(double window) {
+  const unsigned long long w = (unsigned long long)__double_as_longlong(window);
   return w == 0x3ff0000000000000ull ? 1 : ((w & kAbsMask) == 0 ? 0 : 2);
 }
 
@@ -179,11 +179,10 @@ k_hogbom(HogArgs a) {
     unsigned long long bv = 0;
     int bi = kNoPixel;
     const unsigned codes = SMEM && a.window ? s_code[i * 32 + lane] : 0x5555u;
-    auto one = [&](int j) {
+    auto one = [&](int j, double r, double win) {
       const int p = lane + 32 * j;
       const long long c = col + p, px = row * a.ny + c;
       if (c >= a.ny) return;
-      double r = SMEM ? s_res[i * kHogSeg + p] : a.res[px];
       if (prow && c >= c0 && c < c1) {
         r = __dsub_rn(r, __dmul_rn(pre ? pre[j] : prow[c], mval));
         if (SMEM)
@@ -191,15 +190,30 @@ k_hogbom(HogArgs a) {
         else
           a.res[px] = r;
       }
-      const int code = SMEM ? (codes >> (2 * j)) & 3 : (a.window ? hog_code(a.window, px) : 1);
-      const unsigned long long v = hog_value(r, code, a.window + px);
+      const int code = SMEM ? (codes >> (2 * j)) & 3 : hog_code(win);
+      const unsigned long long v = hog_value(r, code, SMEM ? a.window + px : &win);
       if (v != ~0ull) hog_take(v, p, &bv, &bi);
     };
     if (SMEM) {
 #pragma unroll
-      for (int j = 0; j < kHogPx; ++j) one(j);
-    } else {
-      for (int j = 0; j < width / 32; ++j) one(j);
+      for (int j = 0; j < kHogPx; ++j) one(j, s_res[i * kHogSeg + lane + 32 * j], 0.0);
+    } else {  // eight pixels a lane at a time from global memory; the first search copies the image
+      const double *from = prow ? a.res : a.src;
+      for (int j0 = 0; j0 < width / 32; j0 += kHogPx) {
+        double r[kHogPx], win[kHogPx];
+#pragma unroll
+        for (int j = 0; j < kHogPx; ++j) {
+          const long long c = col + lane + 32 * (j0 + j);
+          r[j] = c < a.ny ? from[row * a.ny + c] : 0.0;
+          win[j] = a.window && c < a.ny ? a.window[row * a.ny + c] : 1.0;
+        }
+#pragma unroll
+        for (int j = 0; j < kHogPx; ++j) {
+          const long long c = col + lane + 32 * (j0 + j);
+          if (from != a.res && c < a.ny) a.res[row * a.ny + c] = r[j];
+          one(j0 + j, r[j], win[j]);
+        }
+      }
     }
     if (lane == hog_best_lane(bv, (unsigned)bi)) {
       s_segv[i] = bv;
@@ -218,11 +232,9 @@ k_hogbom(HogArgs a) {
         const long long c = col + lane + 32 * j;
         const bool in = c < a.ny;
         s_res[i * kHogSeg + lane + 32 * j] = in ? a.src[row * a.ny + c] : 0.0;
-        codes |= (in && a.window ? hog_code(a.window, row * a.ny + c) : 1) << (2 * j);
+        codes |= (in && a.window ? hog_code(a.window[row * a.ny + c]) : 1) << (2 * j);
       }
       s_code[i * 32 + lane] = (unsigned short)codes;
-    } else if (a.src != a.res) {
-      for (int p = lane; p < width && col + p < a.ny; p += 32) a.res[row * a.ny + col + p] = a.src[row * a.ny + col + p];
     }
     scan(i, row, col, nullptr, 0, 0, 0.0, nullptr);
   }
