@@ -1944,8 +1944,12 @@ k_grid_own(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__
 // (sum re t.re, sum re t.im) and (sum im t.re, sum im t.im), instead of four.
 // STASH (with a chunk of at most kStashRows rows and a cf table of fewer than
 // 2^31 taps): the footprint pass leaves each row's set-up in shared memory.
-template <typename R, int NPOL, int NW, bool DUP = false, int LPR = 0, int SGC = 0, bool STASH = false>
-__global__ void __launch_bounds__(NW * 32)
+//
+// CTAS: CTAs an SM to leave the registers for, where not 0 (four polarisations: the
+// compiler's own 80 registers give three too, but bounded to three it keeps less of a
+// segment's set-up in them and spills 40 bytes: better where few rows share a bin).
+template <typename R, int NPOL, int NW, bool DUP = false, int LPR = 0, int SGC = 0, bool STASH = false, int CTAS = 0>
+__global__ void __launch_bounds__(NW * 32, CTAS)
 k_degrid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict__ sidx,
               const uint32_t *__restrict__ off, uint32_t chunk, int64_t nvis,
               const typename Cplx<R>::T *__restrict__ cf, const typename Cplx<R>::T *__restrict__ grid,
@@ -3382,8 +3386,13 @@ static int launch_degrid(const Geom &g, const PlanBufs &b, int64_t nvis, const v
         // (Supports above 8: with four rows per warp the set-up is already shared.)
         const bool stash = g.npol == 1 && g.S > 8 && g_tune_stash.load() != 0 &&
                            chunk_rows() <= (uint32_t)kStashRows && cf_elems(g) < 0x7fffffffll;
+        // Four polarisations, S = 8, bounded to three CTAs / not, us: 2 rows a bin 5516 / 11398, 10 6885 / 10695,
+        // 20 7962 / 8188, 30 9239 / 9070, 60 12916 / 12049 (4096^2, 20 slices), 400 3562 / 3143 (2048^2, 5 slices).
         if (g.npol == 4)
-          kern = by_lpr(IntC<4>(), IntC<32>(), BoolC<false>());
+          kern = lpr > 16 || lpr == 0 || nvis >= 24 * (int64_t)g.nbins
+                     ? by_lpr(IntC<4>(), IntC<32>(), BoolC<false>())
+                     : lpr == 8 ? k_degrid_lean<R, 4, kWarps, true, 8, 32, false, 3>
+                                : k_degrid_lean<R, 4, kWarps, true, 16, 32, false, 3>;
         else if (g.npol == 2)
           kern = by_lpr(IntC<2>(), IntC<48>(), BoolC<false>());
         else
