@@ -2308,24 +2308,39 @@ k_degrid_rows(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restric
         tp[u] = gofs[u] >= 0 ? k[8 * u] : czero<CT>();
         gv[u] = gofs[u] >= 0 ? c[gofs[u]] : czero<CT>();
       }
-      R ax = 0, ay = 0;
-      bool real = sizeof(R) == 8;  // FP64, as in k_degrid_lean: two FMAs a tap where this lane's taps are real
-      if constexpr (sizeof(R) == 8) {
+      R ax, ay;
+      if constexpr (sizeof(R) == 4) {  // four sums, as the packed degridder's: two would be chains of sixteen roundings
+        float rr = 0.f, ri = 0.f, ir = 0.f, ii = 0.f;
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u) {
+          rr = fmaf(gv[u].x, tp[u].x, rr);
+          ir = fmaf(gv[u].y, tp[u].x, ir);
+        }
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u) {
+          ii = fmaf(gv[u].y, tp[u].y, ii);
+          ri = fmaf(gv[u].x, tp[u].y, ri);
+        }
+        ax = rr - ii;
+        ay = ri + ir;
+      } else {  // as k_degrid_lean: two FMAs a tap where this lane's taps are real
+        bool real = true;
 #pragma unroll
         for (int u = 0; u < STEPS; ++u)
           real = real && (__double_as_longlong(tp[u].y) << 1) == 0 && finite_bits(gv[u].x) && finite_bits(gv[u].y);
-      }
-      if (real) {
+        ax = ay = 0;
+        if (real) {
 #pragma unroll
-        for (int u = 0; u < STEPS; ++u) {
-          ax = fma(gv[u].x, tp[u].x, ax);
-          ay = fma(gv[u].y, tp[u].x, ay);
-        }
-      } else {
+          for (int u = 0; u < STEPS; ++u) {
+            ax = fma(gv[u].x, tp[u].x, ax);
+            ay = fma(gv[u].y, tp[u].x, ay);
+          }
+        } else {
 #pragma unroll
-        for (int u = 0; u < STEPS; ++u) {
-          ax = fma(gv[u].x, tp[u].x, fma(-gv[u].y, tp[u].y, ax));
-          ay = fma(gv[u].x, tp[u].y, fma(gv[u].y, tp[u].x, ay));
+          for (int u = 0; u < STEPS; ++u) {
+            ax = fma(gv[u].x, tp[u].x, fma(-gv[u].y, tp[u].y, ax));
+            ay = fma(gv[u].x, tp[u].y, fma(gv[u].y, tp[u].x, ay));
+          }
         }
       }
 #pragma unroll
