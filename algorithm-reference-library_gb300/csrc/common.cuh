@@ -99,14 +99,14 @@ struct Geom {
   int32_t SG;      // staged subgrid edge = T + S
   int32_t ntu, ntv;
   uint32_t rcpT;   // ceil(2^32 / T): pixel / T as a high word (exact below 2^20 pixels)
-  uint32_t nbins;  // nchan * nw * ntv * ntu; key == nbins marks a rejected row
+  uint32_t nbins;  // nchan * nw * ntv * ntu; bin nbins holds the rejected rows
 };
 
 int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precision, int64_t nvis, Geom *g);
 
 // Workspace carve-up for a plan over nvis rows.
 struct PlanBufs {
-  uint32_t *keys;     // rank of each row within its bin
+  uint32_t *ranks;    // of each row within its bin
   RowMap *maps;
   uint32_t *sidx;
   RowMap *smap;

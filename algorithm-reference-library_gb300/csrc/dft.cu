@@ -227,8 +227,9 @@ k_dft_predict32(const double *__restrict__ uvw, const int32_t *__restrict__ chan
 // Channel of each row: the rank of its frequency among the rows' distinct ones
 // (get_frequency_map with no image; numpy.unique's order: ascending, NaNs equal
 // and last, the two zeros equal).  A table of at least twice as many slots as
-// the components have channels holds the distinct values; one more value than
-// that is the caller's error, so the table never fills.
+// the components have channels holds the distinct values.  More values than
+// channels are the caller's error; rows that pass the count's check together can
+// fill the table then, so every probe is bounded by its size.
 //   k_chan_first   empties the table and adds the first rows' values: with the
 //                  channel the fastest axis, as rows are ordered, all of them
 //   k_chan_insert  every other row's value (the row that claims a slot counts it)

@@ -1264,7 +1264,7 @@ k_grid_lean(Geom g, const RowMap *__restrict__ smap, const uint32_t *__restrict_
 }
 
 // Bin-order copies of one-polarisation rows' vis and weight for the FP32C
-// gridder.  They go into the plan's mapping scratch (the per-row keys and
+// gridder.  They go into the plan's mapping scratch (the per-row ranks and
 // RowMaps k_map writes for k_scatter), which is dead once the plan is built,
 // so the gridder reads vis and weight contiguously by sorted position instead
 // of gathering them through the sort index inside its row loop.  Copies, not
@@ -2905,8 +2905,8 @@ int make_geom(const arlgpu_grid_desc *gd, const arlgpu_cf_desc *cd, int precisio
                 (g->skip_zg || plane(gd->w, g->rcp_gw, gd->nw, &g->fw)) &&
                 (g->skip_zc || plane(cd->z, g->rcp_cz, cd->nz, &g->fz)) && plane(gd->f, g->rcp_gf, gd->nchan, &g->ff);
   }
-  // Subgrid edge: 64 cells when npol planes of it (with the FP32 compensation
-  // words) fit in 64 KiB of shared memory, else 32.
+  // Subgrid edge: 48 cells when npol planes of it (16 bytes a cell) fit in 64 KiB of shared
+  // memory, else 32; what the caller asks for; or the small one below.
   const size_t cell = precision == ARLGPU_FP64 ? 16 : 16;  // c128, or c64 sum + c64 comp
   int SG = g_tune_subgrid.load();
   auto fitted = [&](int e) {
@@ -2974,7 +2974,7 @@ int plan_carve(void *ws, size_t bytes, int64_t nvis, const Geom &g, PlanBufs *b)
     return fail(ARLGPU_ERR_INVALID, "workspace must start on a 16-byte boundary");
   char *p = static_cast<char *>(ws);
   size_t n = (size_t)nvis;
-  b->keys = reinterpret_cast<uint32_t *>(p);
+  b->ranks = reinterpret_cast<uint32_t *>(p);
   p += align_up(n * 4);
   b->maps = reinterpret_cast<RowMap *>(p);
   p += align_up(n * sizeof(RowMap));
@@ -3009,7 +3009,7 @@ int plan_build(const double *uvw, const double *freq, int64_t nvis, const Geom &
   const unsigned plan_blocks = (unsigned)((nvis + 255) / 256);
   ARL_CUDA(cudaMemsetAsync(b.hist, 0, (size_t)nh * 4, st));
   if (nvis > 0) {
-    k_map<<<plan_blocks, 256, 0, st>>>(uvw, freq, nvis, g, b.keys, b.maps, b.hist);
+    k_map<<<plan_blocks, 256, 0, st>>>(uvw, freq, nvis, g, b.ranks, b.maps, b.hist);
     ARL_LAUNCH_CHECK();
     count_launch(1);
   }
@@ -3033,7 +3033,7 @@ int plan_build(const double *uvw, const double *freq, int64_t nvis, const Geom &
     count_launch(3);
   }
   if (nvis > 0) {
-    k_scatter<<<plan_blocks, 256, 0, st>>>(b.keys, b.maps, nvis, g, b.offsets, b.sidx, b.smap);
+    k_scatter<<<plan_blocks, 256, 0, st>>>(b.ranks, b.maps, nvis, g, b.offsets, b.sidx, b.smap);
     ARL_LAUNCH_CHECK();
     count_launch(1);
   }
@@ -3144,7 +3144,7 @@ static int launch_grid_fx(const Geom &g, const PlanBufs &b, int64_t nvis, const 
   const void *vis_k = vis, *wt_k = wt;
   if (sorted) {
     float2 *vis_s = reinterpret_cast<float2 *>(b.maps);
-    float *wt_s = reinterpret_cast<float *>(b.keys);
+    float *wt_s = reinterpret_cast<float *>(b.ranks);
     const int gblocks = (int)std::min<int64_t>((nvis + 255) / 256, (int64_t)num_sms() * 8);
     k_gather_rows<<<gblocks, 256, 0, st>>>(b.sidx, b.offsets, g.nbins, static_cast<const float2 *>(vis),
                                            static_cast<const float *>(wt), vis_s, wt_s);

@@ -7,7 +7,7 @@
 // for at start-up), and real-time pipelines that allocate everything once
 // when they start and forbid allocation, with its possible implicit
 // synchronisation, afterwards.  For them this file keeps the gridder's
-// scratch (the row plan: mapping, bin keys, sorted row ids, bin histogram and
+// scratch (the row plan: mapping, ranks, sorted row ids, bin histogram and
 // offsets) in a fixed file-scope device array, so the entry point needs
 // nothing beyond the caller's inputs and outputs.
 //
@@ -40,7 +40,7 @@ constexpr int64_t kMaxBins = 1 << 16;  // 65,536 bins per call
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Same carve-up as the workspace of arlgpu_grid (keys, RowMap, sorted ids,
+// Same carve-up as the workspace of arlgpu_grid (ranks, RowMap, sorted ids,
 // sorted RowMap, histogram, offsets) at the maximum sizes above.
 constexpr size_t kScratchBytes = align256(kMaxRows * 4) + align256(kMaxRows * 16) + align256(kMaxRows * 4) +
                                  align256(kMaxRows * 16) + align256((kMaxBins + 1) * 4) +

@@ -95,7 +95,7 @@ unsigned long long arlgpu_kernel_launches(void);
  *                   3 = as 2 without the compensation (measurement only: FP32C
  *                       promises compensated sums, so the autotuner never picks it),
  *                   4 = the default: one warp per tile with a subgrid of its own where that is
- *                       the faster (one support: FP32C with one polarisation, up to 8 taps
+ *                       the faster (one support: FP32C with one polarisation, 4 to 8 taps
  *                       and from 2 Mi rows; FP64 with one or two, up to 10 taps), else FP32C
  *                       tiles summed in two-limb 32-bit fixed point: the rounded
  *                       contributions and their rounding residuals (needs cf tap_absmax; FP64 and an unknown bound use 2),
@@ -103,12 +103,14 @@ unsigned long long arlgpu_kernel_launches(void);
  *   "degrid_kernel" 0 = one warp per row, 1 = 32-row batches per warp,
  *                   2 = one warp per row, specialised on npol, groups of four steps,
  *                   3 = as 2 with the staged cells duplicated (re, re, im, im) so each tap is
- *                       two packed FP32 multiply-adds (default; FP32C, FP64 uses 2),
+ *                       two packed FP32 multiply-adds (default; FP32C, FP64 uses 2); with one
+ *                       polarisation, one support of 4 to 8, subgrids of at most 32 cells and 2 Mi
+ *                       rows, in either precision, eight lanes per row straight from the grid,
  *                   4 = as 3 with the grid tile and each row's kernel taps brought into shared
  *                       memory by TMA tensor copies (FP32C, one polarisation, support <= 32,
  *                       subgrid 48, 16-byte aligned tables, even nx; otherwise 3)
  *   "subgrid"       subgrid edge in cells (16..128), 0 = automatic (48; 32 with more pols than one or with
- *                   one pol, one support up to 8, 2 Mi rows and no more bins than rows)
+ *                   one pol, one support of 4 to 8, 2 Mi rows and no more bins than rows)
  *   "chunk"         sorted rows per gridder / degridder CTA (32..2^20, default 512)
  *   "persistent"    1 = the lean and fixed-point kernels run as one grid of resident CTAs,
  *                   each looping over every gridDim-th chunk; 2 = the same resident grid fed by
@@ -311,7 +313,10 @@ int arlgpu_unpack_rows(const void *records, int64_t nvis, int64_t stride, int32_
  * arlgpu_dft_predict: vis[r][p] += sum_k flux[k][row_chan[r]][p] exp(-2 pi i (u l + v m + w n))
  *   for uvw [nvis][3] (wavelengths), lmn [ncomp][3] = (l, m, sqrt(1-l^2-m^2) - 1), flux
  *   [ncomp][nchan][npol] float64, vis [nvis][npol] complex of the precision (updated in
- *   place).  row_chan [nvis] int32 may be NULL when nchan == 1.  Phases in FP64.
+ *   place).  row_chan [nvis] int32 may be NULL when nchan == 1.  FP64 forms its
+ *   phases in FP64; FP32C modulo one turn in 32-bit fixed point, off by at most 2^-29 turns
+ *   before the rounding to FP32 (in FP64 for rows of 2^31 wavelengths and more and for
+ *   direction cosines outside (-1, 1)).
  * arlgpu_dft_adjoint: image[k][p] += Re sum_r conj(exp(-2 pi i uvw_r . lmn_k)) x[r][p], the
  *   adjoint for one channel (no reference counterpart; the dense gradient reference).
  * arlgpu_row_channels: row_chan[r] = the rank of frequency[r] among the rows' distinct
