@@ -136,7 +136,8 @@ __device__ __forceinline__ double divide(double w, double sum) { return w / sum;
 __device__ __forceinline__ float divide(float w, double sum) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(sum);
   const int e = (int)(b >> 52) & 0x7ff;
-  if (e < 1023 - 60 || e > 1023 + 60 || !(w == 0.f || (fabsf(w) > 1e-18f && fabsf(w) < 1e18f)))
+  // weights from 1e-14 on: a quotient's low part stays a normal FP32 number, or its spacing below 1e-5 of its half ulp
+  if (e < 1023 - 60 || e > 1023 + 60 || !(w == 0.f || (fabsf(w) > 1e-14f && fabsf(w) < 1e18f)))
     return (float)((double)w / sum);
   // sum as hi + lo from its bits: 24 leading bits, then the other 29
   const float hi = __uint_as_float((unsigned)((b >> 63) << 31) | (unsigned)(e - 1023 + 127) << 23 |

@@ -53,3 +53,24 @@ def test_quotients_at_rounding_boundaries(arl, npol):
     w64 = w.astype(numpy.float64)
     want = (w64 / w64.sum(1, keepdims=True)).astype(numpy.float32)
     assert numpy.array_equal(got, numpy.repeat(want.reshape(-1, 1), npol, axis=1))
+
+
+def test_quotients_near_the_smallest_normal(arl):
+    """One heavy and one faint weight a cell: the faint one's quotient is so small that the
+    low part of a double-single one would be a few units of the smallest FP32 number."""
+    rng = numpy.random.default_rng(5)
+    N, cell, n = 128, 2e-3, 14000
+    w = numpy.stack([rng.uniform(1e17, 9e17, n), 10.0 ** rng.uniform(-17.9, -11, n)], 1).astype(numpy.float32)
+    im = arl.create_image(npixel=N, cellsize=cell, frequency=numpy.array([1e8]), channel_bandwidth=numpy.array([1e7]),
+                          phasecentre=arl.PhaseCentre(0.0, -45.0))
+    gcf, cf = arl.create_pswf_convolutionfunction(im, oversampling=8, support=6)
+    at = rng.permutation(120 * 120)[:n]
+    uv = numpy.stack([at % 120 - 60.0, at // 120 - 60.0, numpy.zeros(n)], 1) / (N * cell)
+    vis = arl.DeviceVisibility(torch.as_tensor(numpy.repeat(uv, 2, axis=0), device='cuda'),
+                               torch.full((2 * n,), 1e8, dtype=torch.float64, device='cuda'),
+                               torch.zeros((2 * n, 1), dtype=torch.complex64, device='cuda'),
+                               torch.as_tensor(w.reshape(-1, 1), device='cuda'), im.polarisation_frame, im.phasecentre)
+    got = arl.weight_visibility(vis, im, gcfcf=(gcf, cf)).imaging_weight.cpu().numpy()
+    w64 = w.astype(numpy.float64)
+    want = (w64 / w64.sum(1, keepdims=True)).astype(numpy.float32)
+    assert numpy.array_equal(got, want.reshape(-1, 1))
